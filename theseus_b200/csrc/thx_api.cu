@@ -200,21 +200,20 @@ struct DeviceGuard {
 };
 
 bool pick_order_kernels(thx_operator_s *h, int vk) {
-  const bool ns = h->ns;
   const bool bl = h->blend;
 #define THX_PICK(P, D, NN)                                                  \
   if (h->dim == D && h->N == NN) {                                          \
     auto k = order_kernels_##P##_##D##_##NN();                              \
     const bool tma = h->cfg.volume_staging == 1 && !bl;                    \
     if (P == 0) {                                                           \
-      h->vol64 = reinterpret_cast<VolLaunch<double>>(tma ? k.vol_tma[vk][ns ? 1 : 0]      \
-                                                         : k.vol[vk][ns ? 1 : 0][bl ? 1 : 0]); \
+      h->vol64 = reinterpret_cast<VolLaunch<double>>(tma ? k.vol_tma[vk] : k.vol[vk]); \
+      h->small64 = reinterpret_cast<SmallLaunch<double>>(k.small[vk][h->small > 1]); \
       h->grad64 = reinterpret_cast<GradLaunch<double>>(k.grad);             \
       h->blend64 = reinterpret_cast<BlendLaunch<double>>(k.blend);          \
       h->fv64 = reinterpret_cast<VolLaunch<double>>(k.fv);                  \
     } else {                                                                \
-      h->vol32 = reinterpret_cast<VolLaunch<float>>(tma ? k.vol_tma[vk][ns ? 1 : 0]       \
-                                                        : k.vol[vk][ns ? 1 : 0][bl ? 1 : 0]); \
+      h->vol32 = reinterpret_cast<VolLaunch<float>>(tma ? k.vol_tma[vk] : k.vol[vk]); \
+      h->small32 = reinterpret_cast<SmallLaunch<float>>(k.small[vk][h->small > 1]);  \
       h->grad32 = reinterpret_cast<GradLaunch<float>>(k.grad);              \
       h->blend32 = reinterpret_cast<BlendLaunch<float>>(k.blend);           \
       h->fv32 = reinterpret_cast<VolLaunch<float>>(k.fv);                   \
@@ -398,6 +397,9 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
                : (cfg->volume_flux == THX_FLUX_PIROZZOLI)   ? VOL_PIROZZOLI
                                                             : VOL_CENTRAL;
   h->lte = table != nullptr;
+  h->small = h->lte || (h->mixed && (h->blend || h->nbf > 0)) || cfg->volume_staging == 1 ? 0 : small_mesh(g->dim, h->N, h->ne);
+  // a batched case's last steps: its buffers are those of the batched kernels
+  if (h->pool && h->small > 1) h->small = 1;
   if (h->lte) {
     if (!pick_lte_kernels(h)) return THX_ERR_UNSUPPORTED;
   } else {
@@ -518,16 +520,20 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
   }
   // scratch
   const size_t fsz = (size_t)(h->nf + h->nbf) * h->neq * nfp;
+  // the line volume kernel takes the viscous divergence from the gradient kernel
+  const bool div = h->ns && !h->lte;
   if (h->mixed) {
     float *p;
     if ((st = dev_alloc(&p, fsz, A))) return st;
     h->fstar = p;
     if (h->ns) { if ((st = dev_alloc(&p, (size_t)dim * (h->neq - 1) * h->L, A))) return st; h->vflux = p; }
+    if (div) { if ((st = dev_alloc(&p, (size_t)(h->neq - 1) * h->L, A))) return st; h->vdiv = p; }
   } else {
     double *p;
     if ((st = dev_alloc(&p, fsz, A))) return st;
     h->fstar = p;
     if (h->ns) { if ((st = dev_alloc(&p, (size_t)dim * (h->neq - 1) * h->L, A))) return st; h->vflux = p; }
+    if (div) { if ((st = dev_alloc(&p, (size_t)(h->neq - 1) * h->L, A))) return st; h->vdiv = p; }
     if (h->ns && !h->lte) { if ((st = dev_alloc(&p, (size_t)h->neq * h->L, A))) return st; h->svars = p; }
   }
   if ((st = dev_alloc(&h->status, 1, A))) return st;
@@ -635,6 +641,7 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
     VolArgs<float> va{};
     GradArgs<float> ga{};
     ce = h->vol32(va, 0, 1);
+    if (ce == cudaSuccess && h->small) ce = h->small32(va, FaceArgs<float>{}, 0, 0, 1);
     if (ce == cudaSuccess && h->ns) ce = h->grad32(ga, 0, 1);
     if (ce == cudaSuccess && h->blend) ce = h->fv32(va, 0, 1);
     if (ce == cudaSuccess && h->islands) {
@@ -646,6 +653,7 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
     VolArgs<double> va{};
     GradArgs<double> ga{};
     ce = h->vol64(va, 0, 1);
+    if (ce == cudaSuccess && h->small) ce = h->small64(va, FaceArgs<double>{}, 0, 0, 1);
     if (ce == cudaSuccess && h->ns) ce = h->grad64(ga, 0, 1);
     if (ce == cudaSuccess && h->blend && h->fv64) ce = h->fv64(va, 0, 1);
   }
@@ -675,6 +683,8 @@ Geo<float> geo(thx_operator_s *h, float *) {
 }
 VolLaunch<double> volk(thx_operator_s *h, double *) { return h->vol64; }
 VolLaunch<float> volk(thx_operator_s *h, float *) { return h->vol32; }
+SmallLaunch<double> smallk(thx_operator_s *h, double *) { return h->small64; }
+SmallLaunch<float> smallk(thx_operator_s *h, float *) { return h->small32; }
 EntropyLaunch<double> entk(thx_operator_s *h, double *) { return h->ent64; }
 EntropyLaunch<float> entk(thx_operator_s *h, float *) { return h->ent32; }
 GradLaunch<double> gradk(thx_operator_s *h, double *) { return h->grad64; }
@@ -701,13 +711,13 @@ void op_args(thx_operator_s *h, const R *u, R *du, int stage, double dt, double 
   R *vfl = reinterpret_cast<R *>(h->vflux);
   R *fst = reinterpret_cast<R *>(h->fstar);
   ga = GradArgs<R>{};
-  ga.u = u; ga.vflux = vfl; ga.ne = h->ne;
+  ga.u = u; ga.vflux = vfl; ga.vdiv = reinterpret_cast<R *>(h->vdiv); ga.ne = h->ne;
   ga.jac = G.jac; ga.jac_es = h->lay.jac_es; ga.jac_ns = h->lay.jac_ns;
   ga.met = G.met; ga.met_es = h->lay.met_es; ga.met_ns = h->lay.met_ns;
   ga.elem_face = h->elem_face; ga.face_elem = h->face_elem; ga.face_lface = h->face_lface;
   ga.normal = G.nrm; ga.n_fs = h->lay.n_fs; ga.n_ps = h->lay.n_ps;
   ga.wm = G.wm; ga.wp = G.wp; ga.w_fs = h->lay.w_fs; ga.w_ps = h->lay.w_ps;
-  ga.D = G.D; ga.gas = g; ga.status = h->status;
+  ga.D = G.D; ga.Dhat = G.ops + h->N * h->N; ga.gas = g; ga.status = h->status;
   ga.svars = reinterpret_cast<const R *>(h->svars);
   ga.nf_int = h->nf;
   if constexpr (IsF32<R>::value) {
@@ -730,6 +740,7 @@ void op_args(thx_operator_s *h, const R *u, R *du, int stage, double dt, double 
   va.elem_face = h->elem_face; va.fstar = fst;
   va.wm = G.wm; va.wp = G.wp; va.w_fs = h->lay.w_fs; va.w_ps = h->lay.w_ps;
   va.vflux = vfl;
+  va.vdiv = ga.vdiv;
   va.nf_int = h->nf;
   if constexpr (IsF32<R>::value) va.bw = nullptr;
   else va.bw = h->bdr_w;
@@ -739,7 +750,7 @@ void op_args(thx_operator_s *h, const R *u, R *du, int stage, double dt, double 
   va.fv_flux = h->cfg.fv_flux;
   va.gas = g;
   va.ops = G.ops;
-  va.stage = stage; va.dt = dt; va.um = um; va.y = y; va.yf = yf;
+  va.stage = stage; va.dt = dt; va.um = um; va.y = y; va.yo = y; va.yf = yf;
   for (int k = 0; k < 5; ++k) va.off[k] = IsF32<R>::value ? h->off.v[k] : 0.0;
   va.status = h->status;
 }
@@ -755,6 +766,18 @@ template void op_args<float>(thx_operator_s *, const float *, float *, int, doub
 
 namespace {
 
+// Whether the kernel's results (rate, stage state, working copy) share memory
+// with its input u (n values).
+template <typename R>
+bool result_overlaps(const R *u, const VolArgs<R> &va, long long n) {
+  auto hit = [&](const void *p, size_t size) {
+    const uintptr_t a = (uintptr_t)p, b = (uintptr_t)u;
+    return p && a < b + sizeof(R) * (size_t)n && b < a + size * (size_t)n;
+  };
+  if (va.stage == 0) return va.du64 ? hit(va.du64, 8) : hit(va.du, sizeof(R));
+  return hit(va.stage == 3 ? va.um : va.yo, 8) || hit(va.yf, 4);
+}
+
 // One right-hand side: [T recovery] [indicator] [gradient] face fluxes,
 // volume+lift.  stage 0 writes du; stages 1..3 apply the SSP-RK3 update in place.
 // FP32-mixed: u64 is the FP64 state the working copy u was narrowed from
@@ -762,7 +785,8 @@ namespace {
 template <typename R>
 int run_rhs(thx_operator_s *h, const R *u, R *du, cudaStream_t s, int stage, double dt,
             double *um, double *y, float *yf, cudaEvent_t *ev = nullptr, double *du64 = nullptr,
-            const double *dt_dev = nullptr, const double *u64 = nullptr, bool narrow_in_grad = false) {
+            const double *dt_dev = nullptr, const double *u64 = nullptr, bool narrow_in_grad = false,
+            double *yo = nullptr) {
   R *tag = nullptr;
   if (ev) cudaEventRecord(ev[0], s);
   GradArgs<R> ga;
@@ -771,6 +795,10 @@ int run_rhs(thx_operator_s *h, const R *u, R *du, cudaStream_t s, int stage, dou
   op_args<R>(h, u, du, stage, dt, um, y, yf, ga, fa, va);
   va.du64 = du64;
   va.dt_dev = dt_dev;
+  if (yo) va.yo = yo;
+  // the fused kernel reads its neighbours' states while other CTAs write
+  // their elements' results: not for a result that overlaps the input
+  const int small = h->small > 1 && result_overlaps(u, va, h->L * h->neq) ? 0 : h->small;
   if constexpr (IsF32<R>::value) {
     if (narrow_in_grad) {
       // the gradient kernel narrows the FP64 state into the working copy
@@ -826,6 +854,7 @@ int run_rhs(thx_operator_s *h, const R *u, R *du, cudaStream_t s, int stage, dou
     va64.dt_dev = dt_dev;
     for (int k = 0; k < 5; ++k) va64.off[k] = h->off.v[k];
     va.skip_block = h->isl_flag;
+    va.skip_epb = h->isl_epb;
   }
   if (ev) cudaEventRecord(ev[1], s);
   // FP64 Navier-Stokes (ideal gas): the entropy variables of every node
@@ -835,7 +864,7 @@ int run_rhs(thx_operator_s *h, const R *u, R *du, cudaStream_t s, int stage, dou
     return THX_ERR_CUDA;
   if (h->ns && gradk(h, tag)(ga, s, 0) != cudaSuccess) return THX_ERR_CUDA;
   if (ev) cudaEventRecord(ev[2], s);
-  if (facek(h, tag)(fa, s) != cudaSuccess) return THX_ERR_CUDA;
+  if (small < 2 && facek(h, tag)(fa, s) != cudaSuccess) return THX_ERR_CUDA;
   if (isl && h->isl_face(fa64, h->isl_count + 1, s) != cudaSuccess) return THX_ERR_CUDA;
   if (isl && h->nbf > 0) {
     // boundary faces in FP64 into the islands' face fluxes
@@ -863,10 +892,45 @@ int run_rhs(thx_operator_s *h, const R *u, R *du, cudaStream_t s, int stage, dou
   }
   // the FP32 subcell rate, for blended elements outside the islands
   if (h->blend && !(isl && h->isl_alpha_in) && fvk(h, tag)(va, s, 0) != cudaSuccess) return THX_ERR_CUDA;
-  if (volk(h, tag)(va, s, 0) != cudaSuccess) return THX_ERR_CUDA;
+  if ((small ? smallk(h, tag)(va, fa, h->cfg.surface_flux, s, 0) : volk(h, tag)(va, s, 0)) != cudaSuccess)
+    return THX_ERR_CUDA;
   if (isl && h->isl_vol(va64, h->isl_blocks, h->isl_count, s, 0) != cudaSuccess) return THX_ERR_CUDA;
   if (ev) cudaEventRecord(ev[4], s);
   return THX_OK;
+}
+
+// Buffers of the Runge-Kutta stages.  The fused small-mesh kernel cannot write
+// over the state it reads, so its stages alternate between two.
+int stage_buffers(thx_operator_s *h) {
+  const size_t n = (size_t)h->L * h->neq;
+  int st;
+  if (!h->y && (st = dev_alloc(&h->y, n, h->allocs))) return st;
+  if (h->small > 1 && !h->mixed && !h->y2 && (st = dev_alloc(&h->y2, n, h->allocs))) return st;
+  if (h->small > 1 && h->mixed && !h->yf2 && (st = dev_alloc(&h->yf2, n, h->allocs))) return st;
+  return THX_OK;
+}
+
+// The three SSP-RK3 stages of one step on u; dt_dev (may be null): the step in
+// device memory.  FP32-mixed: cur is the working copy of u, and afterwards
+// that of the new state.
+int rk3_step(thx_operator_s *h, double *u, double dt, const double *dt_dev, float *&cur, cudaStream_t s) {
+  int st;
+  if (h->mixed) {
+    for (int stage = 1; stage <= 3; ++stage) {
+      float *next = h->yf2 ? (cur == h->yf ? h->yf2 : h->yf) : cur;
+      if ((st = run_rhs<float>(h, cur, nullptr, s, stage, dt, u, h->y, next, nullptr, nullptr, dt_dev,
+                               stage == 1 ? u : h->y)))
+        return st;
+      cur = next;
+    }
+    return THX_OK;
+  }
+  double *y2 = h->y2 ? h->y2 : h->y;
+  if ((st = run_rhs<double>(h, u, nullptr, s, 1, dt, u, h->y, nullptr, nullptr, nullptr, dt_dev))) return st;
+  if ((st = run_rhs<double>(h, h->y, nullptr, s, 2, dt, u, h->y, nullptr, nullptr, nullptr, dt_dev, nullptr, false,
+                            y2)))
+    return st;
+  return run_rhs<double>(h, y2, nullptr, s, 3, dt, u, y2, nullptr, nullptr, nullptr, dt_dev);
 }
 
 int check_device() {
@@ -1189,22 +1253,12 @@ int thx_rk3_steps(thx_handle h, double *u, double dt, int nsteps, void *stream) 
   DeviceGuard dg(h->device);
   if (!dg.ok) return THX_ERR_CUDA;
   cudaStream_t s = (cudaStream_t)stream;
-  const long long n = h->L * h->neq;
   int st;
-  if (!h->y && (st = dev_alloc(&h->y, (size_t)n, h->allocs))) return st;
+  if ((st = stage_buffers(h))) return st;
   if (h->mixed && (st = to_working_copy(h, u, s))) return st;
-  for (int step = 0; step < nsteps; ++step) {
-    if (h->mixed) {
-      for (int stage = 1; stage <= 3; ++stage)
-        if ((st = run_rhs<float>(h, h->yf, nullptr, s, stage, dt, u, h->y, h->yf, nullptr, nullptr,
-                                 nullptr, stage == 1 ? u : h->y)))
-          return st;
-    } else {
-      if ((st = run_rhs<double>(h, u, nullptr, s, 1, dt, u, h->y, nullptr))) return st;
-      if ((st = run_rhs<double>(h, h->y, nullptr, s, 2, dt, u, h->y, nullptr))) return st;
-      if ((st = run_rhs<double>(h, h->y, nullptr, s, 3, dt, u, h->y, nullptr))) return st;
-    }
-  }
+  float *cur = h->yf;
+  for (int step = 0; step < nsteps; ++step)
+    if ((st = rk3_step(h, u, dt, nullptr, cur, s))) return st;
   return THX_OK;
 }
 
@@ -1215,26 +1269,17 @@ int thx_rk3_steps_cfl(thx_handle h, double *u, double cfl, int nsteps, double *d
   DeviceGuard dg(h->device);
   if (!dg.ok) return THX_ERR_CUDA;
   cudaStream_t s = (cudaStream_t)stream;
-  const long long n = h->L * h->neq;
   int st;
-  if (!h->y && (st = dev_alloc(&h->y, (size_t)n, h->allocs))) return st;
+  if ((st = stage_buffers(h))) return st;
   if (h->mixed && (st = to_working_copy(h, u, s))) return st;
+  float *cur = h->yf;
   for (int step = 0; step < nsteps; ++step) {
     // dt from the stability rates of the step's initial state, on the device
     if ((st = stability_rates(h, u, s))) return st;
     cfl_dt_kernel<<<1, 1, 0, s>>>(h->stab, cfl, h->dtd, dt_history ? dt_history + step : nullptr,
                                   h->status);
     if (cudaGetLastError() != cudaSuccess) return THX_ERR_CUDA;
-    if (h->mixed) {
-      for (int stage = 1; stage <= 3; ++stage)
-        if ((st = run_rhs<float>(h, h->yf, nullptr, s, stage, 0.0, u, h->y, h->yf, nullptr, nullptr,
-                                 h->dtd, stage == 1 ? u : h->y)))
-          return st;
-    } else {
-      if ((st = run_rhs<double>(h, u, nullptr, s, 1, 0.0, u, h->y, nullptr, nullptr, nullptr, h->dtd))) return st;
-      if ((st = run_rhs<double>(h, h->y, nullptr, s, 2, 0.0, u, h->y, nullptr, nullptr, nullptr, h->dtd))) return st;
-      if ((st = run_rhs<double>(h, h->y, nullptr, s, 3, 0.0, u, h->y, nullptr, nullptr, nullptr, h->dtd))) return st;
-    }
+    if ((st = rk3_step(h, u, 0.0, h->dtd, cur, s))) return st;
   }
   return THX_OK;
 }
@@ -1277,10 +1322,10 @@ int thx_rk3_time_loop(thx_handle h, double *u, double cfl, int ncycles, thx_time
   DeviceGuard dg(h->device);
   if (!dg.ok) return THX_ERR_CUDA;
   cudaStream_t s = (cudaStream_t)stream;
-  const long long n = h->L * h->neq;
   int st;
-  if (!h->y && (st = dev_alloc(&h->y, (size_t)n, h->allocs))) return st;
+  if ((st = stage_buffers(h))) return st;
   if (h->mixed && (st = to_working_copy(h, u, s))) return st;
+  float *cur = h->yf;
   const bool variable = cfl > 0.0;
   if (variable) {
     if ((st = stability_rates(h, u, s))) return st;
@@ -1289,16 +1334,7 @@ int thx_rk3_time_loop(thx_handle h, double *u, double cfl, int ncycles, thx_time
   for (int c = 0; c < ncycles; ++c) {
     time_loop_begin_kernel<<<1, 1, 0, s>>>(loop, h->dtd, dt_history ? dt_history + c : nullptr);
     if (cudaGetLastError() != cudaSuccess) return THX_ERR_CUDA;
-    if (h->mixed) {
-      for (int stage = 1; stage <= 3; ++stage)
-        if ((st = run_rhs<float>(h, h->yf, nullptr, s, stage, 0.0, u, h->y, h->yf, nullptr, nullptr,
-                                 h->dtd, stage == 1 ? u : h->y)))
-          return st;
-    } else {
-      if ((st = run_rhs<double>(h, u, nullptr, s, 1, 0.0, u, h->y, nullptr, nullptr, nullptr, h->dtd))) return st;
-      if ((st = run_rhs<double>(h, h->y, nullptr, s, 2, 0.0, u, h->y, nullptr, nullptr, nullptr, h->dtd))) return st;
-      if ((st = run_rhs<double>(h, h->y, nullptr, s, 3, 0.0, u, h->y, nullptr, nullptr, nullptr, h->dtd))) return st;
-    }
+    if ((st = rk3_step(h, u, 0.0, h->dtd, cur, s))) return st;
     if (variable && (st = stability_rates(h, u, s))) return st;
     time_loop_end_kernel<<<1, 1, 0, s>>>(loop, h->dtd, h->stab, cfl, h->status);
     if (cudaGetLastError() != cudaSuccess) return THX_ERR_CUDA;

@@ -286,6 +286,8 @@ __device__ __forceinline__ void bc_viscous(const GasT<double> &g, const thx_bc &
 
 template <int DIM, int SURF, bool NS>
 __global__ void __launch_bounds__(128) bnd_face_kernel(const BndArgs a) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int NEQ = DIM + 2;
   const int N = a.N;
   const int nfp = DIM == 2 ? N : N * N;

@@ -68,12 +68,18 @@ __device__ __forceinline__ float rexp(float x) { return expf(x); }
 template <typename R> __device__ __forceinline__ R rabs(R x) { return x < R(0) ? -x : x; }
 template <typename R> __device__ __forceinline__ R rmax(R a, R b) { return a > b ? a : b; }
 
+// How the logarithmic mean is formed: by the branch, or by its near-equal
+// series alone (the caller knows that the arguments take it), so that no
+// branch separates the means of several pairs in flight.
+enum LogMeanMode { LM_BRANCH = 0, LM_SERIES = 1 };
+
 // include/theseus_kernels.hpp:106-123.  In FP32 the series branch (equal
 // arguments, where the closed form cancels) is evaluated in FP64.
+template <int MODE = LM_BRANCH>
 __device__ __forceinline__ double log_mean(double x, double y) {
   const double xi = y / x;
   const double u = (xi * (xi - 2.0) + 1.0) / (xi * (xi + 2.0) + 1.0);
-  if (u < 1e-4) {
+  if (MODE == LM_SERIES || u < 1e-4) {
     const double denom = 105.0 + u * (35.0 + u * (21.0 + 15.0 * u));
     return (x + y) * 52.5 / denom;
   }
@@ -86,11 +92,12 @@ __device__ __forceinline__ double log_mean(double x, double y) {
 // with eps = u (35 + u (21 + 15 u)) / 105 <= 3.4e-5, 52.5 / (105 (1 + eps)) =
 // (1 - eps + eps^2) / 2 to a relative 4e-14, far below the FP32 result's
 // rounding, without an FP64 division.
+template <int MODE = LM_BRANCH>
 __device__ __forceinline__ float log_mean(float x, float y) {
   const float s = x + y, d = y - x;
   const float f = fdiv(d, s);
   const float u = f * f;
-  if (u < 1e-4f) {
+  if (MODE == LM_SERIES || u < 1e-4f) {
     const double ud = u;
     const double eps = ud * (35.0 + ud * (21.0 + 15.0 * ud)) * (1.0 / 105.0);
     return s * (float)(0.5 * (1.0 - eps + eps * eps));
@@ -211,12 +218,13 @@ __device__ __forceinline__ R mom_p(const R *a) {
 // (f^2 = u; terms through u^6, truncation below 5e-9), so the deviation is
 // (d1+d2)/2 - ((x1+x2)/2) (S-1)/S with no cancellation; beyond, the closed
 // form, whose deviation is formed by difference.
+template <int MODE>
 __device__ __forceinline__ void log_mean_dev(float x1, float x2, float d1, float d2, float xr,
                                              float &val, float &dev) {
   const float s = x1 + x2, d = x2 - x1;
   const float f = fdiv(d, s);
   const float u = f * f;
-  if (u < 0.0625f) {
+  if (MODE == LM_SERIES || u < 0.0625f) {
     const float sm1 =
         u * (1.f / 3.f + u * (1.f / 5.f + u * (1.f / 7.f + u * (1.f / 9.f + u * (1.f / 11.f + u * (1.f / 13.f))))));
     const float mean = 0.5f * s;
@@ -237,12 +245,12 @@ __device__ __forceinline__ void log_mean_dev(float x1, float x2, float d1, float
 // with dp_hat = ((drho1+drho2)/2 - p_r (dbeta1+dbeta2)) / (beta1+beta2) and
 // dh_hat = -dbeta_ln g1/(2 beta_ln beta_r) + v_r.dvbar + |dvbar|^2
 //          - (|dv1|^2 + |dv2|^2)/4 + (dp_hat rho_r - p_r drho_ln)/(rho_ln rho_r).
-template <int DIM>
+template <int DIM, int MODE>
 __device__ __forceinline__ void vol_chandrashekar_pert(const GasT<float> &g, const float *a, const float *b,
                                                        const float *met, float *F) {
   float rho_ln, drho_ln, beta_ln, dbeta_ln;
-  log_mean_dev(a[0], b[0], a[DIM + 3], b[DIM + 3], g.rho_r, rho_ln, drho_ln);
-  log_mean_dev(a[DIM + 1], b[DIM + 1], a[DIM + 2], b[DIM + 2], g.beta_r, beta_ln, dbeta_ln);
+  log_mean_dev<MODE>(a[0], b[0], a[DIM + 3], b[DIM + 3], g.rho_r, rho_ln, drho_ln);
+  log_mean_dev<MODE>(a[DIM + 1], b[DIM + 1], a[DIM + 2], b[DIM + 2], g.beta_r, beta_ln, dbeta_ln);
   float dvb[DIM], vb[DIM];
   float dvn = 0.f, vnr = 0.f, vrdv = 0.f, dv2 = 0.f, dvs = 0.f;
 #pragma unroll
@@ -269,18 +277,19 @@ __device__ __forceinline__ void vol_chandrashekar_pert(const GasT<float> &g, con
 }
 
 // ---- two-point volume fluxes (metric rows already averaged) --------------
+// MODE: how their logarithmic means branch.
 // include/ChandrashekarFlux.hpp:20-89
-template <typename R, int DIM>
+template <typename R, int DIM, int MODE = LM_BRANCH>
 __device__ __forceinline__ void vol_chandrashekar(const GasT<R> &g, const R *a, const R *b,
                                                   const R *met, R *F) {
   if constexpr (IsF32<R>::value) {
     if (g.pert) {
-      vol_chandrashekar_pert<DIM>(g, a, b, met, F);
+      vol_chandrashekar_pert<DIM, MODE>(g, a, b, met, F);
       return;
     }
   }
   const R rho1 = a[0], rho2 = b[0];
-  const R rho_ln = log_mean(rho1, rho2);
+  const R rho_ln = log_mean<MODE>(rho1, rho2);
   R mom_hat[DIM];
   R h_hat = R(0), vn = R(0);
 #pragma unroll
@@ -292,7 +301,7 @@ __device__ __forceinline__ void vol_chandrashekar(const GasT<R> &g, const R *a, 
     h_hat += -R(0.25) * (v1 * v1 + v2 * v2) + vbar * vbar;
   }
   const R beta1 = a[DIM + 2], beta2 = b[DIM + 2];
-  const R beta_ln = log_mean(beta1, beta2);
+  const R beta_ln = log_mean<MODE>(beta1, beta2);
   const R p_hat = fdiv(R(0.5) * (rho1 + rho2), beta1 + beta2);
   h_hat += fdiv(R(0.5), beta_ln) * g.gm1_av_inv + fdiv(p_hat, rho_ln);
   // FP32: p_hat - p_ref = (beta1 pp1 + beta2 pp2)/(beta1 + beta2), exactly
@@ -305,11 +314,11 @@ __device__ __forceinline__ void vol_chandrashekar(const GasT<R> &g, const R *a, 
 }
 
 // include/RanochaFlux.hpp:20-79
-template <typename R, int DIM>
+template <typename R, int DIM, int MODE = LM_BRANCH>
 __device__ __forceinline__ void vol_ranocha(const GasT<R> &g, const R *a, const R *b,
                                             const R *met, R *F) {
   const R rho1 = a[0], rho2 = b[0];
-  const R rho_ln = log_mean(rho1, rho2);
+  const R rho_ln = log_mean<MODE>(rho1, rho2);
   const R p1 = a[DIM + 1], p2 = b[DIM + 1];
   const R pbar = R(0.5) * (p1 + p2);
   R vbar[DIM];
@@ -322,7 +331,7 @@ __device__ __forceinline__ void vol_ranocha(const GasT<R> &g, const R *a, const 
     ke += R(0.5) * (v1 * v2);
     fe += (R(0.5) * (p1 * v2 + p2 * v1)) * met[d];
   }
-  const R inv_beta_ln = fdiv(p1 * p2, log_mean(rho1 * p2, rho2 * p1));
+  const R inv_beta_ln = fdiv(p1 * p2, log_mean<MODE>(rho1 * p2, rho2 * p1));
   const R ie = inv_beta_ln * g.inv_gm1;
   const R p_mom = IsF32<R>::value ? R(0.5) * (mom_p<R, DIM>(a) + mom_p<R, DIM>(b)) : pbar;
   F[0] = rho_ln * vn;

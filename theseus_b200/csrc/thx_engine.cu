@@ -50,6 +50,7 @@ size_t case_bytes(const thx_geometry *g, const thx_config *cfg, int flow) {
   if (mixed) b += round_up(L * neq * 4);                      // FP32 working copy
   b += round_up(nf * nfp * neq * s);                          // face fluxes
   if (ns) b += round_up((size_t)dim * (neq - 1) * L * s);     // viscous flux
+  if (ns) b += round_up((neq - 1) * L * s);                   // its divergence
   b += round_up(L * gs) + round_up(L * dim * dim * gs);       // J, metric
   b += round_up(nf * nfp * dim * gs) + 2 * round_up(nf * nfp * gs);  // normals, lift weights
   b += round_up(nf * 2 * 4) * 2 + round_up(ne * 2 * dim * 4); // connectivity
@@ -930,11 +931,11 @@ void Engine<double>::pick_kernels(Group<double> &G, int vk, int ns) {
 #define THX_PICKB(P, D, NN)                                 \
   if (G.dim == D && G.N == NN) {                            \
     const OrderKernels0 k = order_kernels_##P##_##D##_##NN(); \
-    G.volb = k.volb[vk][ns];                                \
+    G.volb = k.volb[vk];                                \
     G.gradb = k.gradb;                                      \
     G.epb_full = k.epb;                                     \
     G.epb_half = k.epb_half;                                \
-    G.volb_half = k.volb_half[vk][ns];                      \
+    G.volb_half = k.volb_half[vk];                      \
     G.gradb_half = k.gradb_half;                            \
   }
   THX_FOR_ORDERS(THX_PICKB, 0, 2)
@@ -949,11 +950,11 @@ void Engine<float>::pick_kernels(Group<float> &G, int vk, int ns) {
 #define THX_PICKB(P, D, NN)                                 \
   if (G.dim == D && G.N == NN) {                            \
     const OrderKernels1 k = order_kernels_##P##_##D##_##NN(); \
-    G.volb = k.volb[vk][ns];                                \
+    G.volb = k.volb[vk];                                \
     G.gradb = k.gradb;                                      \
     G.epb_full = k.epb;                                     \
     G.epb_half = k.epb_half;                                \
-    G.volb_half = k.volb_half[vk][ns];                      \
+    G.volb_half = k.volb_half[vk];                      \
     G.gradb_half = k.gradb_half;                            \
   }
   THX_FOR_ORDERS(THX_PICKB, 1, 2)

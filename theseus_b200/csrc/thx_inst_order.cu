@@ -19,30 +19,17 @@ namespace thx {
 THX_TYPE(THX_PREC) THX_NAME(THX_PREC, THX_DIM, THX_N)() {
   using R = THX_RT(THX_PREC);
   THX_TYPE(THX_PREC) k;
-  k.vol[VOL_CHANDRASHEKAR][0][0] = &launch_volume<R, THX_DIM, THX_N, VOL_CHANDRASHEKAR, false, false>;
-  k.vol[VOL_CHANDRASHEKAR][0][1] = &launch_volume<R, THX_DIM, THX_N, VOL_CHANDRASHEKAR, false, true>;
-  k.vol[VOL_CHANDRASHEKAR][1][0] = &launch_volume<R, THX_DIM, THX_N, VOL_CHANDRASHEKAR, true, false>;
-  k.vol[VOL_CHANDRASHEKAR][1][1] = &launch_volume<R, THX_DIM, THX_N, VOL_CHANDRASHEKAR, true, true>;
-  k.vol[VOL_RANOCHA][0][0] = &launch_volume<R, THX_DIM, THX_N, VOL_RANOCHA, false, false>;
-  k.vol[VOL_RANOCHA][0][1] = &launch_volume<R, THX_DIM, THX_N, VOL_RANOCHA, false, true>;
-  k.vol[VOL_RANOCHA][1][0] = &launch_volume<R, THX_DIM, THX_N, VOL_RANOCHA, true, false>;
-  k.vol[VOL_RANOCHA][1][1] = &launch_volume<R, THX_DIM, THX_N, VOL_RANOCHA, true, true>;
-  k.vol[VOL_PIROZZOLI][0][0] = &launch_volume<R, THX_DIM, THX_N, VOL_PIROZZOLI, false, false>;
-  k.vol[VOL_PIROZZOLI][0][1] = &launch_volume<R, THX_DIM, THX_N, VOL_PIROZZOLI, false, true>;
-  k.vol[VOL_PIROZZOLI][1][0] = &launch_volume<R, THX_DIM, THX_N, VOL_PIROZZOLI, true, false>;
-  k.vol[VOL_PIROZZOLI][1][1] = &launch_volume<R, THX_DIM, THX_N, VOL_PIROZZOLI, true, true>;
-  k.vol[VOL_CENTRAL][0][0] = &launch_volume<R, THX_DIM, THX_N, VOL_CENTRAL, false, false>;
-  k.vol[VOL_CENTRAL][0][1] = &launch_volume<R, THX_DIM, THX_N, VOL_CENTRAL, false, true>;
-  k.vol[VOL_CENTRAL][1][0] = &launch_volume<R, THX_DIM, THX_N, VOL_CENTRAL, true, false>;
-  k.vol[VOL_CENTRAL][1][1] = &launch_volume<R, THX_DIM, THX_N, VOL_CENTRAL, true, true>;
-#define THX_SETT(V)                                                              \
-  k.vol_tma[V][0] = &launch_volume_tma<R, THX_DIM, THX_N, V, false>;             \
-  k.vol_tma[V][1] = &launch_volume_tma<R, THX_DIM, THX_N, V, true>;
-  THX_SETT(VOL_CHANDRASHEKAR)
-  THX_SETT(VOL_RANOCHA)
-  THX_SETT(VOL_PIROZZOLI)
-  THX_SETT(VOL_CENTRAL)
-#undef THX_SETT
+#define THX_SETV(V)                                           \
+  k.vol[V] = &launch_volume_line<R, THX_DIM, THX_N, V>;        \
+  k.small[V][0] = &launch_volume_small<R, THX_DIM, THX_N, V, false>; \
+  k.small[V][1] = &launch_volume_small<R, THX_DIM, THX_N, V, true>;  \
+  k.vol_tma[V] = &launch_volume_tma<R, THX_DIM, THX_N, V>;     \
+  k.volb[V] = &launch_volume_batched<R, THX_DIM, THX_N, V>;
+  THX_SETV(VOL_CHANDRASHEKAR)
+  THX_SETV(VOL_RANOCHA)
+  THX_SETV(VOL_PIROZZOLI)
+  THX_SETV(VOL_CENTRAL)
+#undef THX_SETV
 #if THX_PREC == 0
   k.grad = &launch_grad_sv<R, THX_DIM, THX_N>;  // FP64: entropy variables precomputed
 #else
@@ -50,25 +37,14 @@ THX_TYPE(THX_PREC) THX_NAME(THX_PREC, THX_DIM, THX_N)() {
 #endif
   k.blend = &launch_blend<R, THX_DIM, THX_N>;
   k.fv = &launch_fv<R, THX_DIM, THX_N>;
-#define THX_SETB(V)                                                              \
-  k.volb[V][0] = &launch_volume_batched<R, THX_DIM, THX_N, V, false>;             \
-  k.volb[V][1] = &launch_volume_batched<R, THX_DIM, THX_N, V, true>;
-  THX_SETB(VOL_CHANDRASHEKAR)
-  THX_SETB(VOL_RANOCHA)
-  THX_SETB(VOL_PIROZZOLI)
-  THX_SETB(VOL_CENTRAL)
-#undef THX_SETB
   k.gradb = &launch_grad_batched<R, THX_DIM, THX_N>;
   k.epb = Shape<THX_DIM, THX_N>::EPB;
   k.epb_half = half_epb<THX_DIM, THX_N>();
-  for (auto &row : k.volb_half)
-    for (auto &v : row) v = nullptr;
+  for (auto &v : k.volb_half) v = nullptr;
   k.gradb_half = nullptr;
   if constexpr (half_epb<THX_DIM, THX_N>() > 0) {
     constexpr int H = half_epb<THX_DIM, THX_N>();
-#define THX_SETH(V)                                                                \
-  k.volb_half[V][0] = &launch_volume_batched<R, THX_DIM, THX_N, V, false, H>;      \
-  k.volb_half[V][1] = &launch_volume_batched<R, THX_DIM, THX_N, V, true, H>;
+#define THX_SETH(V) k.volb_half[V] = &launch_volume_batched<R, THX_DIM, THX_N, V, H>;
     THX_SETH(VOL_CHANDRASHEKAR)
     THX_SETH(VOL_RANOCHA)
     THX_SETH(VOL_PIROZZOLI)

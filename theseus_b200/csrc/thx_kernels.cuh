@@ -105,6 +105,19 @@ __device__ __forceinline__ unsigned dynamic_smem_bytes() {
   return v;
 }
 
+// Programmatic dependent launch: a kernel launched with launch_early may start
+// while the kernel before it on the stream still runs, and waits here, before
+// it touches memory that kernels write, until that one has completed and its
+// writes are visible (no-op after an ordinary launch).  grid_release lets the
+// next kernel's launch begin as soon as every CTA of this grid has started, so
+// that launch latency and set-up overlap this kernel.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_start() {
+  grid_release();
+  grid_wait();
+}
+
 // Shared-memory layout of the volume kernel, in elements of R:
 // [ops | prim + pair fluxes, or the viscous flux | state (NEEDQ) | metric].
 template <typename R, int DIM, int N, int VOL, bool NS, bool BLEND, int EPBX = 0>
@@ -141,6 +154,7 @@ struct VolArgs {
   int nf_int;             // faces at or past nf_int are boundary faces
   const R *bw;            // boundary lift weights [b][fp], face slot nf_int + b
   const R *vflux;         // NS physical viscous flux [dir][eq-1][elem][node]
+  const R *vdiv;          // NS divergence of the viscous flux [eq-1][elem][node] (line kernel)
   const double *alpha;    // per-element blending coefficient or nullptr
   const R *sub[3];        // subcell metrics (reference layout), element stride sub_es
   long long sub_es[3];
@@ -153,13 +167,15 @@ struct VolArgs {
   double dt;
   const double *dt_dev;   // when set, the stage's dt is read here (device-side CFL step)
   double *um;             // FP64 master state (read every stage, written by stage 3)
-  double *y;              // FP64 stage state (written by stages 1 and 2)
+  double *y;              // FP64 stage state (read by stages 2 and 3)
+  double *yo;             // where stages 1 and 2 write it (y, or another buffer)
   float *yf;              // FP32 working copy of the next RHS input (mixed mode) or nullptr
   double off[5];          // yf = (float)(y - off[eq])
   unsigned *status;
   // FP32-mixed with FP64 islands: blocks (of EPB elements) flagged here are
   // evaluated by the FP64 kernels instead; this kernel skips them
   const int *skip_block;
+  int skip_epb;  // elements per flagged block
 };
 
 // Surface flux with a run-time selector (used on subcell faces).  Inlined:
@@ -512,7 +528,7 @@ __device__ __forceinline__ void volume_body(const VolArgs<R> &a, const int block
       if (a.stage == 3) {
         if (!(a.dt_dev && dt == 0.0)) a.um[i] = ynew[k];
       } else {
-        a.y[i] = ynew[k];
+        a.yo[i] = ynew[k];
       }
       if (a.yf) a.yf[i] = (float)(ynew[k] - a.off[k]);
     }
@@ -621,6 +637,7 @@ __device__ __forceinline__ void fv_body(const VolArgs<R> &a, const int block) {
 
 template <typename R, int DIM, int N>
 __global__ void __launch_bounds__(Shape<DIM, N>::THREADS) fv_kernel(const VolArgs<R> a) {
+  grid_start();
   fv_body<R, DIM, N>(a, blockIdx.x);
 }
 
@@ -634,8 +651,13 @@ __global__ void __launch_bounds__(Shape<DIM, N>::THREADS) volume_kernel(const Vo
 // compiler gives it the whole register file and one CTA).
 template <typename R, int DIM, int N, int VOL, bool NS, bool BLEND, int MINB>
 __global__ void __launch_bounds__(Shape<DIM, N>::THREADS, MINB) volume_kernel_mb(const VolArgs<R> a) {
+  grid_start();
   volume_body<R, DIM, N, VOL, NS, BLEND>(a, blockIdx.x);
 }
+
+}  // namespace thx
+#include "thx_volume.cuh"
+namespace thx {
 
 // ---- TMA-staged volume kernel ---------------------------------------------
 // Persistent CTAs walk the element blocks; while a CTA evaluates one block,
@@ -697,16 +719,13 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned by
       : "memory");
 }
 
-template <typename R, int DIM, int N, int VOL, bool NS, bool BLEND>
+template <typename R, int DIM, int N, int VOL>
 struct VolTmaSmem {
   using S = Shape<DIM, N>;
-  static constexpr size_t base(bool metric_per_node) {
-    return (VolSmem<R, DIM, N, VOL, NS, BLEND>::bytes(metric_per_node) + 15) / 16 * 16;
-  }
+  static constexpr int T = line_threads<DIM, N, S::EPB>();
+  static constexpr size_t base = (LineSmem<R, DIM, N, VOL, T, S::EPB>::bytes() + 15) / 16 * 16;
   static constexpr size_t buf_elems = (size_t)S::NEQ * stage_kstride<R, DIM, N>();
-  static constexpr size_t bytes(bool metric_per_node) {
-    return base(metric_per_node) + 2 * buf_elems * sizeof(R) + 2 * sizeof(unsigned long long);
-  }
+  static constexpr size_t bytes = base + 2 * buf_elems * sizeof(R) + 2 * sizeof(unsigned long long);
 };
 
 // Thread 0: stage block `blk` into buffer `dst` (bulk copies counted on bar),
@@ -732,19 +751,18 @@ __device__ __forceinline__ bool tma_stage_issue(const VolArgs<R> &a, int blk, R 
   return true;
 }
 
-template <typename R, int DIM, int N, int VOL, bool NS, bool BLEND, int MINB>
-__global__ void __launch_bounds__(Shape<DIM, N>::THREADS, MINB > 0 ? MINB : 1)
+template <typename R, int DIM, int N, int VOL>
+__global__ void __launch_bounds__(VolTmaSmem<R, DIM, N, VOL>::T)
 volume_tma_kernel(const VolArgs<R> a) {
   using S = Shape<DIM, N>;
-  using T_ = VolTmaSmem<R, DIM, N, VOL, NS, BLEND>;
+  using T_ = VolTmaSmem<R, DIM, N, VOL>;
   constexpr int ND = S::ND, NEQ = S::NEQ, EPB = S::EPB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const bool mpn = a.met_ns != 0;
-  if (dynamic_smem_bytes() < T_::bytes(mpn)) {
+  if (dynamic_smem_bytes() < T_::bytes) {
     if (threadIdx.x == 0) atomicOr(a.status, STATUS_LAUNCH);
     return;
   }
-  R *buf0 = reinterpret_cast<R *>(smem_raw + T_::base(mpn));
+  R *buf0 = reinterpret_cast<R *>(smem_raw + T_::base);
   R *bufs[2] = {buf0, buf0 + T_::buf_elems};
   unsigned long long *bars = reinterpret_cast<unsigned long long *>(buf0 + 2 * T_::buf_elems);
   __shared__ int s_bulk[2];  // buffer staged by bulk copy (1) or to be loaded (0)
@@ -789,7 +807,7 @@ volume_tma_kernel(const VolArgs<R> a) {
       phase[b] ^= 1u;
       pending[b] = false;
     }
-    volume_body<R, DIM, N, VOL, NS, BLEND>(a, blk, bufs[b]);
+    volume_line_body<R, DIM, N, VOL, T_::T, S::EPB>(a, blk, bufs[b], stage_kstride<R, DIM, N>());
     __syncthreads();  // shared memory and the buffer are free for the next block
   }
   if (s_fail) {
@@ -823,21 +841,19 @@ struct FaceArgs {
   const int *order;
 };
 
-// Face point t (face order[t / nfp], point t % nfp) of one case.
+// Flux F* of point fp of face f (minus to plus side).  SURF < 0: the surface
+// flux is chosen at run time (kind).
 template <typename R, int DIM, int SURF, bool NS>
-__device__ __forceinline__ void face_body(const FaceArgs<R> &a, const long long t) {
+__device__ __forceinline__ void face_point_flux(const FaceArgs<R> &a, const int f, const int fp, R *F,
+                                                const int kind = 0) {
   constexpr int NEQ = DIM + 2;
   const int N = a.N;
-  const int nfp = DIM == 2 ? N : N * N;
   const int nd = DIM == 2 ? N * N : N * N * N;
-  if (t >= (long long)a.nf * nfp) return;
-  const int fi = (int)(t / nfp), fp = (int)(t % nfp);
-  const int f = a.order ? a.order[fi] : fi;
   const long long L = (long long)a.ne * nd;
   const int em = a.face_elem[2 * f], ep = a.face_elem[2 * f + 1];
   const long long im = (long long)em * nd + trace_node<DIM>(N, a.face_lface[2 * f], fp);
   const long long ip = (long long)ep * nd + trace_node<DIM>(N, a.face_lface[2 * f + 1], fp);
-  R qm[NEQ], qp[NEQ], nrm[DIM], F[NEQ];
+  R qm[NEQ], qp[NEQ], nrm[DIM];
 #pragma unroll
   for (int k = 0; k < NEQ; ++k) { qm[k] = a.u[k * L + im]; qp[k] = a.u[k * L + ip]; }
   const R *np = a.normal + ((long long)f * a.n_fs + (long long)fp * a.n_ps) * DIM;
@@ -855,7 +871,8 @@ __device__ __forceinline__ void face_body(const FaceArgs<R> &a, const long long 
     FState<R, DIM> A, B;
     make_fstate<R, DIM>(a.gas, qm, A);
     make_fstate<R, DIM>(a.gas, qp, B);
-    surface_flux<R, DIM, SURF>(a.gas, A, B, nrm, F);
+    if constexpr (SURF < 0) surface_flux_rt<R, DIM>(kind, a.gas, A, B, nrm, F);
+    else surface_flux<R, DIM, SURF>(a.gas, A, B, nrm, F);
   }
   if (NS) {
     // include/DGSEMIntegrator.hpp:261-316: F* -= n . avg(F_v), with the physical
@@ -870,9 +887,25 @@ __device__ __forceinline__ void face_body(const FaceArgs<R> &a, const long long 
         F[1 + k] -= nrm[d] * (R(0.5) * (vm + vp));
       }
   }
+}
+
+// Face point t (face order[t / nfp], point t % nfp) of one case.
+template <typename R, int DIM, int SURF, bool NS>
+__device__ __forceinline__ void face_body(const FaceArgs<R> &a, const long long t) {
+  constexpr int NEQ = DIM + 2;
+  const int nfp = DIM == 2 ? a.N : a.N * a.N;
+  if (t >= (long long)a.nf * nfp) return;
+  const int fi = (int)(t / nfp), fp = (int)(t % nfp);
+  const int f = a.order ? a.order[fi] : fi;
+  R F[NEQ];
+  face_point_flux<R, DIM, SURF, NS>(a, f, fp, F);
 #pragma unroll
   for (int k = 0; k < NEQ; ++k) a.fstar[((long long)f * NEQ + k) * nfp + fp] = F[k];
 }
+
+}  // namespace thx
+#include "thx_small.cuh"
+namespace thx {
 
 // The face kernels: one thread per face point, each precision compiled for
 // its own number of resident 128-thread CTAs per SM.  FP64: eight (64
@@ -882,10 +915,12 @@ __device__ __forceinline__ void face_body(const FaceArgs<R> &a, const long long 
 // compiler's 62 at eight).
 template <int DIM, int SURF, bool NS>
 __global__ void __launch_bounds__(128, 8) face_kernel_f64(const FaceArgs<double> a) {
+  grid_start();
   face_body<double, DIM, SURF, NS>(a, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 template <int DIM, int SURF, bool NS>
 __global__ void __launch_bounds__(128, 10) face_kernel_f32(const FaceArgs<float> a) {
+  grid_start();
   face_body<float, DIM, SURF, NS>(a, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -895,6 +930,7 @@ __global__ void __launch_bounds__(128, 10) face_kernel_f32(const FaceArgs<float>
 // p=4: 0.244 -> 0.208 ms; three CTAs, 168 registers: 0.215 ms).
 template <int DIM, bool NS>
 __global__ void __launch_bounds__(128, 4) face_kernel_lte(const FaceArgs<double> a) {
+  grid_start();
   face_body<double, DIM, SURF_LTEEC, NS>(a, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -903,6 +939,7 @@ template <typename R>
 struct GradArgs {
   const R *u;
   R *vflux;   // physical viscous flux [dir][eq-1][elem][node] (mass row omitted)
+  R *vdiv;    // its weak-form divergence [eq-1][elem][node] (not scaled by 1/J), or nullptr
   int ne;
   const R *jac;
   long long jac_es, jac_ns;
@@ -914,6 +951,7 @@ struct GradArgs {
   const R *wm, *wp;
   long long w_fs, w_ps;
   const R *D;  // N*N
+  const R *Dhat;  // N*N, weak form (vdiv)
   GasT<R> gas;
   const R *svars;  // entropy variables of every node [eq][elem][node] (SV kernels)
   unsigned *status;
@@ -937,10 +975,59 @@ struct GradArgs {
   double off[5];
 };
 
+__host__ __device__ constexpr size_t max_of(size_t x, size_t y) { return x > y ? x : y; }
+
+// Weak-form divergence with Dhat of the physical viscous flux vf[pd*NV + k]
+// of the thread's node (include/DGSEMIntegrator.hpp:486-622): contravariant
+// fluxes through shared memory, sDh the operator, sFv [EPB][DIM][NV][ND].
+// Every thread of the CTA calls it; the region sFv may be in use before.
+template <typename R, int DIM, int N, int EPBX = 0>
+__device__ __forceinline__ void viscous_divergence(const GradArgs<R> &a, const R *sDh, R *sFv, const R *vf,
+                                                   const R *row, const int el, const int n, const int e,
+                                                   const bool active) {
+  using S = Shape<DIM, N, EPBX>;
+  constexpr int ND = S::ND, NV = S::NEQ - 1;
+  __syncthreads();
+  if (active) {
+#pragma unroll
+    for (int dir = 0; dir < DIM; ++dir)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        R f = R(0);
+#pragma unroll
+        for (int pd = 0; pd < DIM; ++pd) f += row[dir * DIM + pd] * vf[pd * NV + k];
+        sFv[((el * DIM + dir) * NV + k) * ND + n] = f;
+      }
+  }
+  __syncthreads();
+  if (!active) return;
+  int c[3];
+  node_coords<DIM, N>(n, c);
+  R dv[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) dv[k] = R(0);
+#pragma unroll
+  for (int dir = 0; dir < DIM; ++dir) {
+    const int me = c[dir];
+    const int line = line_of<DIM, N>(dir, c);
+#pragma unroll
+    for (int l = 0; l < N; ++l) {
+      const int s = line_node<DIM, N>(dir, line, l);
+      const R co = sDh[me * N + l];
+#pragma unroll
+      for (int k = 0; k < NV; ++k) dv[k] += co * sFv[((el * DIM + dir) * NV + k) * ND + s];
+    }
+  }
+  const long long L = (long long)a.ne * ND;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) a.vdiv[k * L + (long long)e * ND + n] = dv[k];
+}
+
 template <typename R, int DIM, int N, int EPBX = 0>
 __host__ __device__ constexpr size_t grad_smem_bytes() {
   using S = Shape<DIM, N, EPBX>;
-  return sizeof(R) * (S::DPAD + (size_t)S::EPB * S::NEQ * (S::ND + 2 * DIM * S::NFP));
+  return sizeof(R) * (2 * S::DPAD + S::EPB * max_of((size_t)S::NEQ * (S::ND + 2 * DIM * S::NFP),
+                                                   (size_t)DIM * (S::NEQ - 1) * S::ND));
 }
 
 // Entropy variables of every node (include/EOS.hpp:206-234, as
@@ -951,6 +1038,7 @@ __host__ __device__ constexpr size_t grad_smem_bytes() {
 template <typename R, int DIM>
 __global__ void __launch_bounds__(256) entropy_kernel(const R *__restrict__ u, long long L,
                                                       const GasT<R> gas, R *__restrict__ sv) {
+  grid_start();
   constexpr int NEQ = DIM + 2;
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= L) return;
@@ -975,14 +1063,18 @@ __device__ __forceinline__ void grad_body(const GradArgs<R> &a, const int block)
   constexpr int ND = S::ND, NEQ = S::NEQ, EPB = S::EPB, NFP = S::NFP, NLF = 2 * DIM;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R *sD = reinterpret_cast<R *>(smem_raw);   // N*N (padded)
-  R *sS = sD + S::DPAD;                      // [EPB][NEQ][ND] own entropy variables
+  R *sDh = sD + S::DPAD;                     // N*N (padded)
+  R *sS = sDh + S::DPAD;                     // [EPB][NEQ][ND] own entropy variables
   R *sN = sS + EPB * NEQ * ND;               // [EPB][2*DIM][NEQ][NFP] neighbour traces
   if (dynamic_smem_bytes() < grad_smem_bytes<R, DIM, N, EPBX>()) {
     if (threadIdx.x == 0 && a.status) atomicOr(a.status, STATUS_LAUNCH);
     return;
   }
   const int tid = threadIdx.x;
-  for (int i = tid; i < N * N; i += blockDim.x) sD[i] = a.D[i];
+  for (int i = tid; i < N * N; i += blockDim.x) {
+    sD[i] = a.D[i];
+    sDh[i] = a.Dhat[i];
+  }
   const int el = tid / ND, n = tid % ND;
   const int e0 = block * EPB;
   const int e = e0 + el;
@@ -1053,7 +1145,9 @@ __device__ __forceinline__ void grad_body(const GradArgs<R> &a, const int block)
     for (int k = 0; k < NEQ; ++k) sN[((tel * NLF + lf) * NEQ + k) * NFP + fp] = so[k];
   }
   __syncthreads();
-  if (!active) return;
+  constexpr int NV = NEQ - 1;
+  R vfs[DIM * NV];  // physical viscous flux of the node [dir][eq-1]
+  auto node = [&]() {
   int c[3];
   node_coords<DIM, N>(n, c);
   R dref[DIM][NEQ];
@@ -1181,12 +1275,13 @@ __device__ __forceinline__ void grad_body(const GradArgs<R> &a, const int block)
     for (int cc = 0; cc < DIM; ++cc) grad_entropy_to_prim_ng<R, DIM>(ng, q, g[cc], dp + cc * NEQ);
     viscous_flux_ng<R, DIM>(a.gas, q, ng, dp, vf);
   }
-  constexpr int NV = NEQ - 1;
 #pragma unroll
   for (int d = 0; d < DIM; ++d)
 #pragma unroll
-    for (int k = 0; k < NV; ++k)
-      a.vflux[((long long)d * NV + k) * L + (long long)e * ND + n] = vf[(1 + k) * DIM + d];
+    for (int k = 0; k < NV; ++k) {
+      vfs[d * NV + k] = vf[(1 + k) * DIM + d];
+      a.vflux[((long long)d * NV + k) * L + (long long)e * ND + n] = vfs[d * NV + k];
+    }
   // primitive gradients at this node's boundary points, for the viscous
   // boundary fluxes
   if constexpr (!IsF32<R>::value && !LTE) {
@@ -1203,18 +1298,24 @@ __device__ __forceinline__ void grad_body(const GradArgs<R> &a, const int block)
       }
     }
   }
+  };
+  if (active) node();
+  if (a.vdiv)
+    viscous_divergence<R, DIM, N, EPBX>(a, sDh, sS, vfs, a.met + (long long)e * a.met_es + (long long)n * a.met_ns,
+                                        el, n, e, active);
 }
 
 // Shared memory of the gradient kernel that reads precomputed entropy
-// variables: D | own entropy variables [EPB][NEQ][ND] | own conserved state
+// variables: D | Dhat | own entropy variables [EPB][NEQ][ND] | own conserved state
 // [EPB][NEQ][ND] | lift data [EPB][2*DIM][NEQ+1+DIM][NFP] (the jump -- or the
 // boundary flux --, the weight and the normal of every face point) | face
 // kinds [EPB][2*DIM] (0 none, 1 interior, 2 boundary).
 template <typename R, int DIM, int N>
 __host__ __device__ constexpr size_t grad_sv_smem_bytes() {
   using S = Shape<DIM, N>;
-  return sizeof(R) * (S::DPAD + 2 * (size_t)S::EPB * S::NEQ * S::ND +
-                      (size_t)S::EPB * 2 * DIM * (S::NEQ + 1 + DIM) * S::NFP) +
+  return sizeof(R) * (2 * S::DPAD + S::EPB * max_of(2 * (size_t)S::NEQ * S::ND +
+                                                       (size_t)2 * DIM * (S::NEQ + 1 + DIM) * S::NFP,
+                                                   (size_t)DIM * (S::NEQ - 1) * S::ND)) +
          sizeof(int) * (size_t)S::EPB * 2 * DIM;
 }
 
@@ -1235,7 +1336,8 @@ __device__ __forceinline__ void grad_body_sv(const GradArgs<R> &a, const int blo
   constexpr int NJ = NEQ + 1 + DIM;  // jump, weight, normal per face point
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R *sD = reinterpret_cast<R *>(smem_raw);   // N*N (padded)
-  R *sS = sD + S::DPAD;                      // [EPB][NEQ][ND]
+  R *sDh = sD + S::DPAD;                     // N*N (padded)
+  R *sS = sDh + S::DPAD;                     // [EPB][NEQ][ND]
   R *sQ = sS + EPB * NEQ * ND;               // [EPB][NEQ][ND]
   R *sJ = sQ + EPB * NEQ * ND;               // [EPB][NLF][NJ][NFP]
   int *sK = reinterpret_cast<int *>(sJ + EPB * NLF * NJ * NFP);  // [EPB][NLF]
@@ -1244,7 +1346,10 @@ __device__ __forceinline__ void grad_body_sv(const GradArgs<R> &a, const int blo
     return;
   }
   const int tid = threadIdx.x;
-  for (int i = tid; i < N * N; i += blockDim.x) sD[i] = a.D[i];
+  for (int i = tid; i < N * N; i += blockDim.x) {
+    sD[i] = a.D[i];
+    sDh[i] = a.Dhat[i];
+  }
   const int el = tid / ND, n = tid % ND;
   const int e0 = block * EPB;
   const int e = e0 + el;
@@ -1317,7 +1422,9 @@ __device__ __forceinline__ void grad_body_sv(const GradArgs<R> &a, const int blo
     for (int cc = 0; cc < DIM; ++cc) dst[(NEQ + 1 + cc) * NFP] = nr[cc];
   }
   __syncthreads();
-  if (!active) return;
+  constexpr int NV = NEQ - 1, E = DIM + 1;
+  R vfs[DIM * NV];  // physical viscous flux of the node [dir][eq-1]
+  auto node = [&]() {
   int c[3];
   node_coords<DIM, N>(n, c);
   const R *adj = a.met + (long long)e * a.met_es + (long long)n * a.met_ns;
@@ -1401,7 +1508,6 @@ __device__ __forceinline__ void grad_body_sv(const GradArgs<R> &a, const int blo
     for (int k = 0; k < NEQ; ++k) g[cc][k] = dpc[k];
   }
   const R *dp = &g[0][0];  // dp[d*NEQ + eq]
-  constexpr int NV = NEQ - 1, E = DIM + 1;
   const long long base = (long long)e * ND + n;
   {
     const R mu = viscosity_ng<R, DIM>(a.gas, ng);
@@ -1421,9 +1527,11 @@ __device__ __forceinline__ void grad_body_sv(const GradArgs<R> &a, const int blo
         if (mom == dir) tau = mu * (R(2) * dp[dir * NEQ + 1 + mom] - a.gas.mu_bulk * div);
         else tau = mu * (dp[dir * NEQ + 1 + mom] + dp[mom * NEQ + 1 + dir]);
         a.vflux[((long long)dir * NV + mom) * L + base] = tau;
+        vfs[dir * NV + mom] = tau;
         ef += ng.v[mom] * tau;
       }
       a.vflux[((long long)dir * NV + DIM) * L + base] = ef;
+      vfs[dir * NV + DIM] = ef;
     }
   }
   // primitive gradients at this node's boundary points, for the viscous
@@ -1441,10 +1549,17 @@ __device__ __forceinline__ void grad_body_sv(const GradArgs<R> &a, const int blo
       }
     }
   }
+  };
+  if (active) node();
+  // the staged variables, state and lift factors are no longer needed
+  if (a.vdiv)
+    viscous_divergence<R, DIM, N>(a, sDh, sS, vfs, a.met + (long long)e * a.met_es + (long long)n * a.met_ns, el, n,
+                                  e, active);
 }
 
 template <typename R, int DIM, int N, bool LTE, bool SV = false>
 __global__ void __launch_bounds__(Shape<DIM, N>::THREADS) grad_kernel(const GradArgs<R> a) {
+  grid_start();
   grad_body<R, DIM, N, LTE, SV, 0, IsF32<R>::value>(a, blockIdx.x);
 }
 
@@ -1453,6 +1568,7 @@ __global__ void __launch_bounds__(Shape<DIM, N>::THREADS) grad_kernel(const Grad
 // p=4 (four CTAs, 64 registers with heavier spills: 0.243 ms).
 template <int DIM, int N>
 __global__ void __launch_bounds__(Shape<DIM, N>::THREADS, 3) grad_kernel_lte(const GradArgs<double> a) {
+  grid_start();
   grad_body<double, DIM, N, true, false>(a, blockIdx.x);
 }
 
@@ -1460,6 +1576,7 @@ __global__ void __launch_bounds__(Shape<DIM, N>::THREADS, 3) grad_kernel_lte(con
 // three CTAs per SM (four spill about 230 bytes per thread at 64 registers).
 template <typename R, int DIM, int N>
 __global__ void __launch_bounds__(Shape<DIM, N>::THREADS, 3) grad_sv_kernel(const GradArgs<R> a) {
+  grid_start();
   grad_body_sv<R, DIM, N>(a, blockIdx.x);
 }
 
@@ -1470,6 +1587,7 @@ __global__ void __launch_bounds__(Shape<DIM, N>::THREADS, 3) grad_sv_kernel(cons
 template <int DIM>
 __global__ void __launch_bounds__(256, 2) lte_temperature_kernel(const double *u, long long L, LteDev t,
                                                               double *Tn, int *Cn, unsigned *status) {
+  grid_start();
   constexpr int NEQ = DIM + 2;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < L; i += stride) {
@@ -1598,6 +1716,7 @@ template <typename R, int DIM, int N>
 __global__ void __launch_bounds__(32 * kBlendWarps) blend_warp_kernel(const BlendArgs<R> a,
                                                                       const int *__restrict__ list,
                                                                       const int *__restrict__ count) {
+  grid_start();
   using S = Shape<DIM, N>;
   constexpr int ND = S::ND;
   __shared__ double sV[N * N];
@@ -1624,6 +1743,7 @@ struct Offsets { double v[5]; };
 template <int DIM>
 static __global__ void to_working(long long L, const double *__restrict__ src, float *__restrict__ dst,
                                   Offsets off, double gm1, unsigned *status) {
+  grid_start();
   constexpr int NEQ = DIM + 2;
   const long long stride = (long long)gridDim.x * blockDim.x;
   bool bad = false;
@@ -1726,6 +1846,7 @@ struct StabArgs {
 
 template <int DIM>
 __global__ void stability_kernel(const StabArgs a) {
+  grid_start();
   constexpr int NEQ = DIM + 2;
   const int N = a.N;
   const int nd = DIM == 2 ? N * N : N * N * N;
@@ -1855,6 +1976,7 @@ __global__ void stability_kernel(const StabArgs a) {
 // the numerics flag and dt = 0.
 static __global__ void cfl_dt_kernel(const unsigned long long *rates, double cfl, double *dt, double *history,
                               unsigned *status) {
+  grid_start();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const double adv = __longlong_as_double((long long)rates[0]);
   const double sur = __longlong_as_double((long long)rates[1]);
@@ -1889,16 +2011,14 @@ __device__ __forceinline__ void stage_record(unsigned char *dst, const A *src) {
   for (int i = threadIdx.x; i < (int)(sizeof(A) / 8); i += blockDim.x) d[i] = s[i];
 }
 
-// The batched volume kernel is compiled for four resident 256-thread CTAs per
-// SM (eight of the half-size CTAs): 64 registers a thread.  Bounded to the
-// FP32 one-case kernel's six CTAs (40 registers) its persistent loop spills
-// about 100 bytes per thread and runs 4-8 % slower (2-D).
+// Line kernel over a work list; EPBX (0: Shape's) elements per work item.
 template <typename R, int DIM, int N, int EPBX>
-constexpr int vol_batch_min_blocks() {
-  return 4 * Shape<DIM, N>::THREADS / Shape<DIM, N, EPBX>::THREADS;
+constexpr int line_batch_threads() {
+  return line_threads<DIM, N, Shape<DIM, N, EPBX>::EPB>();
 }
-template <typename R, int DIM, int N, int VOL, bool NS, int EPBX = 0>
-__global__ void __launch_bounds__(Shape<DIM, N, EPBX>::THREADS, (vol_batch_min_blocks<R, DIM, N, EPBX>()))
+template <typename R, int DIM, int N, int VOL, int EPBX = 0>
+__global__ void __launch_bounds__((line_batch_threads<R, DIM, N, EPBX>()),
+                                  (line_min_blocks<R, N, line_batch_threads<R, DIM, N, EPBX>()>()))
 volume_batched(const VolArgs<R> *__restrict__ args, const BatchWork *__restrict__ work,
                const int *__restrict__ nwork) {
   __shared__ __align__(16) unsigned char sa[sizeof(VolArgs<R>)];
@@ -1908,7 +2028,8 @@ volume_batched(const VolArgs<R> *__restrict__ args, const BatchWork *__restrict_
     const BatchWork it = work[w];
     stage_record(sa, &args[it.item]);
     __syncthreads();
-    volume_body<R, DIM, N, VOL, NS, false, EPBX>(*reinterpret_cast<const VolArgs<R> *>(sa), it.block);
+    volume_line_body<R, DIM, N, VOL, line_batch_threads<R, DIM, N, EPBX>(), Shape<DIM, N, EPBX>::EPB>(
+        *reinterpret_cast<const VolArgs<R> *>(sa), it.block);
   }
 }
 
@@ -1985,12 +2106,13 @@ static __global__ void island_faces_kernel(int nf, int epb, const int *__restric
 }
 
 template <typename R, int DIM, int N, int VOL>
-__global__ void __launch_bounds__(Shape<DIM, N>::THREADS, 4)
+__global__ void __launch_bounds__((line_batch_threads<R, DIM, N, 0>()),
+                                  (line_min_blocks<R, N, line_batch_threads<R, DIM, N, 0>()>()))
 volume_list_kernel(const VolArgs<R> a, const int *__restrict__ list, const int *__restrict__ count) {
   const int n = *count;
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
     __syncthreads();  // the previous block's shared memory is free
-    volume_body<R, DIM, N, VOL, false, true>(a, list[w]);
+    volume_line_body<R, DIM, N, VOL, line_batch_threads<R, DIM, N, 0>(), Shape<DIM, N>::EPB>(a, list[w]);
   }
 }
 

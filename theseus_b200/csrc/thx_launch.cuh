@@ -11,6 +11,30 @@ namespace thx {
 using PREC_T_0 = double;
 using PREC_T_1 = float;
 
+// Launch, with programmatic stream serialization (grid_start in the kernel)
+// while the grid is small: there the launch latency is most of the time (RK3
+// stage of the 32^2 p=3 vortex 9.8 -> 7.8 us).  CTAs of a large grid placed
+// early take the SMs that the kernel before has left first, several on one,
+// and the rest of the chip then waits for those (96^2 p=3 FP32-mixed 18.6 ->
+// 27.1 us with the line kernel placed early).
+constexpr unsigned kEarlyGrid = 5 * 148;
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = grid <= kEarlyGrid ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
 template <typename R> using VolLaunch = cudaError_t (*)(const VolArgs<R> &, cudaStream_t, int prepare);
 template <typename R> using FaceLaunch = cudaError_t (*)(const FaceArgs<R> &, cudaStream_t);
 template <typename R> using GradLaunch = cudaError_t (*)(const GradArgs<R> &, cudaStream_t, int prepare);
@@ -49,41 +73,62 @@ cudaError_t launch_volume(const VolArgs<R> &a, cudaStream_t s, int prepare) {
   if (a.ne <= 0) return cudaSuccess;
   const size_t smem = volume_smem_bytes<R, DIM, N, VOL, NS, BLEND>(a.met_ns != 0);
   const int grid = (a.ne + S::EPB - 1) / S::EPB;
-  if constexpr (MINB > 0) volume_kernel_mb<R, DIM, N, VOL, NS, BLEND, MINB><<<grid, S::THREADS, smem, s>>>(a);
+  if constexpr (MINB > 0) return launch_early(volume_kernel_mb<R, DIM, N, VOL, NS, BLEND, MINB>, grid, S::THREADS, smem, s, a);
   else volume_kernel<R, DIM, N, VOL, NS, BLEND><<<grid, S::THREADS, smem, s>>>(a);
   return cudaGetLastError();
 }
 
+// The line kernel (ideal gas): one thread per tensor line.
+template <typename R, int DIM, int N, int VOL, int T = kLineThreads>
+cudaError_t launch_volume_line(const VolArgs<R> &a, cudaStream_t s, int prepare) {
+  using S = LineShape<DIM, N, T>;
+  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T>::bytes();
+  if (prepare)
+    return cudaFuncSetAttribute(volume_line_kernel<R, DIM, N, VOL, T>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (a.ne <= 0) return cudaSuccess;
+  volume_line_kernel<R, DIM, N, VOL, T><<<(a.ne + S::EPB - 1) / S::EPB, T, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+// Small meshes: volume and face terms in one launch (surf: the surface flux).
+template <typename R>
+using SmallLaunch = cudaError_t (*)(const VolArgs<R> &, const FaceArgs<R> &, int surf, cudaStream_t, int prepare);
+
+template <typename R, int DIM, int N, int VOL, bool FACES>
+cudaError_t launch_volume_small(const VolArgs<R> &a, const FaceArgs<R> &fa, int surf, cudaStream_t s, int prepare) {
+  using M = SmallSmem<R, DIM, N, VOL, FACES>;
+  const int epb = small_epb(DIM, N, a.ne);
+  static_assert(M::bytes(small_epb(DIM, N, 1 << 30)) <= 200 * 1024, "shared memory");
+  if (prepare)
+    return cudaFuncSetAttribute(volume_small_kernel<R, DIM, N, VOL, FACES>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)M::bytes(small_epb(DIM, N, 1 << 30)));
+  if (a.ne <= 0) return cudaSuccess;
+  return launch_early(volume_small_kernel<R, DIM, N, VOL, FACES>, (a.ne + epb - 1) / epb, kSmallThreads, M::bytes(epb), s, a, fa, surf, epb);
+}
+
 // Persistent, bulk-copy-staged volume kernel (no blending): as many CTAs as
 // fit on the device at once, each walking the element blocks.
-template <typename R, int DIM, int N, int VOL, bool NS>
+template <typename R, int DIM, int N, int VOL>
 cudaError_t launch_volume_tma(const VolArgs<R> &a, cudaStream_t s, int prepare) {
   using S = Shape<DIM, N>;
-  using T_ = VolTmaSmem<R, DIM, N, VOL, NS, false>;
-  constexpr int MINB = VolMinBlocks<R, VOL, false>::value;
-  auto kern = volume_tma_kernel<R, DIM, N, VOL, NS, false, MINB>;
-  static int cap[2] = {0, 0};  // resident CTAs on the device: metric per element / per node
+  using T_ = VolTmaSmem<R, DIM, N, VOL>;
+  auto kern = volume_tma_kernel<R, DIM, N, VOL>;
+  static int cap = 0;  // resident CTAs on the device
   if (prepare) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)T_::bytes(true));
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T_::bytes);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0;
+    int dev = 0, sms = 0, per = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    for (int m = 0; m < 2; ++m) {
-      int per = 0;
-      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, S::THREADS, T_::bytes(m == 1))) !=
-          cudaSuccess)
-        return e;
-      cap[m] = (per > 0 ? per : 1) * sms;
-    }
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, T_::T, T_::bytes)) != cudaSuccess) return e;
+    cap = (per > 0 ? per : 1) * sms;
     return cudaSuccess;
   }
   if (a.ne <= 0) return cudaSuccess;
-  const int m = a.met_ns != 0 ? 1 : 0;
   const int nblocks = (a.ne + S::EPB - 1) / S::EPB;
-  const int grid = std::min(nblocks, cap[m] > 0 ? cap[m] : 148);
-  kern<<<grid, S::THREADS, T_::bytes(a.met_ns != 0), s>>>(a);
+  kern<<<std::min(nblocks, cap > 0 ? cap : 148), T_::T, T_::bytes, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -93,10 +138,9 @@ cudaError_t launch_face(const FaceArgs<R> &a, cudaStream_t s) {
   const long long total = (long long)a.nf * nfp;
   if (total <= 0) return cudaSuccess;
   const int grid = (int)((total + 127) / 128);
-  if constexpr (SURF == SURF_LTEEC) face_kernel_lte<DIM, NS><<<grid, 128, 0, s>>>(a);
-  else if constexpr (IsF32<R>::value) face_kernel_f32<DIM, SURF, NS><<<grid, 128, 0, s>>>(a);
-  else face_kernel_f64<DIM, SURF, NS><<<grid, 128, 0, s>>>(a);
-  return cudaGetLastError();
+  if constexpr (SURF == SURF_LTEEC) return launch_early(face_kernel_lte<DIM, NS>, grid, 128, 0, s, a);
+  else if constexpr (IsF32<R>::value) return launch_early(face_kernel_f32<DIM, SURF, NS>, grid, 128, 0, s, a);
+  else return launch_early(face_kernel_f64<DIM, SURF, NS>, grid, 128, 0, s, a);
 }
 
 template <typename R, int DIM, int N, bool LTE = false>
@@ -108,16 +152,15 @@ cudaError_t launch_grad(const GradArgs<R> &a, cudaStream_t s, int prepare) {
       return cudaFuncSetAttribute(grad_kernel_lte<DIM, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem);
     if (a.ne <= 0) return cudaSuccess;
-    grad_kernel_lte<DIM, N><<<(a.ne + S::EPB - 1) / S::EPB, S::THREADS, smem, s>>>(a);
+    return launch_early(grad_kernel_lte<DIM, N>, (a.ne + S::EPB - 1) / S::EPB, S::THREADS, smem, s, a);
   } else {
     if (prepare)
       return cudaFuncSetAttribute(grad_kernel<R, DIM, N, LTE>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (a.ne <= 0) return cudaSuccess;
     const int grid = (a.ne + S::EPB - 1) / S::EPB;
-    grad_kernel<R, DIM, N, LTE><<<grid, S::THREADS, smem, s>>>(a);
+    return launch_early(grad_kernel<R, DIM, N, LTE>, grid, S::THREADS, smem, s, a);
   }
-  return cudaGetLastError();
 }
 
 // Gradient from precomputed entropy variables (a.svars, entropy_kernel).
@@ -131,8 +174,7 @@ cudaError_t launch_grad_sv(const GradArgs<R> &a, cudaStream_t s, int prepare) {
   if (a.ne <= 0) return cudaSuccess;
   if (!a.svars) return cudaErrorInvalidValue;
   const int grid = (a.ne + S::EPB - 1) / S::EPB;
-  grad_sv_kernel<R, DIM, N><<<grid, S::THREADS, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_early(grad_sv_kernel<R, DIM, N>, grid, S::THREADS, smem, s, a);
 }
 
 template <typename R>
@@ -141,8 +183,7 @@ using EntropyLaunch = cudaError_t (*)(const R *, long long, const GasT<R> &, R *
 template <typename R, int DIM>
 cudaError_t launch_entropy(const R *u, long long L, const GasT<R> &g, R *sv, cudaStream_t s) {
   if (L <= 0) return cudaSuccess;
-  entropy_kernel<R, DIM><<<(unsigned)((L + 255) / 256), 256, 0, s>>>(u, L, g, sv);
-  return cudaGetLastError();
+  return launch_early(entropy_kernel<R, DIM>, (unsigned)((L + 255) / 256), 256, 0, s, u, L, g, sv);
 }
 
 template <int DIM>
@@ -150,20 +191,21 @@ cudaError_t launch_lte_temperature(const double *u, long long L, const LteDev &t
                                    int *Cn, unsigned *status, cudaStream_t s) {
   if (L <= 0) return cudaSuccess;
   const int grid = (int)std::min<long long>((L + 255) / 256, 148LL * 8);
-  lte_temperature_kernel<DIM><<<grid, 256, 0, s>>>(u, L, t, Tn, Cn, status);
-  return cudaGetLastError();
+  return launch_early(lte_temperature_kernel<DIM>, grid, 256, 0, s, u, L, t, Tn, Cn, status);
 }
 
-template <typename R, int DIM, int N, int VOL, bool NS, int EPBX = 0>
+template <typename R, int DIM, int N, int VOL, int EPBX = 0>
 cudaError_t launch_volume_batched(const VolArgs<R> *args, const BatchWork *work, const int *nwork,
                                   int grid, cudaStream_t s, int prepare) {
-  using S = Shape<DIM, N, EPBX>;
-  constexpr size_t smem = VolSmem<R, DIM, N, VOL, NS, false, EPBX>::bytes(true);
+  constexpr int T = line_batch_threads<R, DIM, N, EPBX>();
+  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T, Shape<DIM, N, EPBX>::EPB>::bytes();
   if (prepare)
-    return cudaFuncSetAttribute(volume_batched<R, DIM, N, VOL, NS, EPBX>,
+    return cudaFuncSetAttribute(volume_batched<R, DIM, N, VOL, EPBX>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (grid <= 0) return cudaSuccess;
-  volume_batched<R, DIM, N, VOL, NS, EPBX><<<grid, S::THREADS, smem, s>>>(args, work, nwork);
+  // the tuned grid counts CTAs of Shape's threads; this kernel's are smaller
+  constexpr int scale = Shape<DIM, N, EPBX>::THREADS / T;
+  volume_batched<R, DIM, N, VOL, EPBX><<<grid * scale, T, smem, s>>>(args, work, nwork);
   return cudaGetLastError();
 }
 
@@ -208,13 +250,12 @@ constexpr int kIslandGrid = 148 * 4;
 template <typename R, int DIM, int N, int VOL>
 cudaError_t launch_volume_list(const VolArgs<R> &a, const int *list, const int *count, cudaStream_t s,
                                int prepare) {
-  using S = Shape<DIM, N>;
-  const int bytes = (int)volume_smem_bytes<R, DIM, N, VOL, false, true>(true);
+  constexpr int T = line_batch_threads<R, DIM, N, 0>();
+  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T, Shape<DIM, N>::EPB>::bytes();
   if (prepare)
     return cudaFuncSetAttribute(volume_list_kernel<R, DIM, N, VOL>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  const size_t smem = volume_smem_bytes<R, DIM, N, VOL, false, true>(a.met_ns != 0);
-  volume_list_kernel<R, DIM, N, VOL><<<kIslandGrid, S::THREADS, smem, s>>>(a, list, count);
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  volume_list_kernel<R, DIM, N, VOL><<<kIslandGrid, T, smem, s>>>(a, list, count);
   return cudaGetLastError();
 }
 
@@ -232,8 +273,7 @@ cudaError_t launch_fv_list(const VolArgs<R> &a, const int *list, const int *coun
 
 template <typename R, int DIM, int N>
 cudaError_t launch_blend_list(const BlendArgs<R> &a, const int *list, const int *count, cudaStream_t s) {
-  blend_warp_kernel<R, DIM, N><<<kIslandGrid, 32 * kBlendWarps, 0, s>>>(a, list, count);
-  return cudaGetLastError();
+  return launch_early(blend_warp_kernel<R, DIM, N>, kIslandGrid, 32 * kBlendWarps, 0, s, a, list, count);
 }
 
 template <typename R, int DIM, int SURF>
@@ -249,8 +289,7 @@ cudaError_t launch_bnd(const BndArgs &a, cudaStream_t s) {
   const int nfp = DIM == 2 ? a.N : a.N * a.N;
   const long long total = (long long)a.nbf * nfp;
   if (total <= 0) return cudaSuccess;
-  bnd_face_kernel<DIM, SURF, NS><<<(unsigned)((total + 127) / 128), 128, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_early(bnd_face_kernel<DIM, SURF, NS>, (unsigned)((total + 127) / 128), 128, 0, s, a);
 }
 
 template <typename R, int DIM, int N>
@@ -261,30 +300,29 @@ cudaError_t launch_fv(const VolArgs<R> &a, cudaStream_t s, int prepare) {
     return cudaFuncSetAttribute(fv_kernel<R, DIM, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (a.ne <= 0 || !a.alpha || !a.fvrate) return cudaSuccess;
   const int grid = (a.ne + S::EPB - 1) / S::EPB;
-  fv_kernel<R, DIM, N><<<grid, S::THREADS, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_early(fv_kernel<R, DIM, N>, grid, S::THREADS, smem, s, a);
 }
 
 template <typename R, int DIM, int N>
 cudaError_t launch_blend(const BlendArgs<R> &a, cudaStream_t s) {
   if (a.ne <= 0) return cudaSuccess;
   const int grid = (a.ne + kBlendWarps - 1) / kBlendWarps;  // one warp per element
-  blend_warp_kernel<R, DIM, N><<<grid, 32 * kBlendWarps, 0, s>>>(a, nullptr, nullptr);
-  return cudaGetLastError();
+  return launch_early(blend_warp_kernel<R, DIM, N>, grid, 32 * kBlendWarps, 0, s, a, nullptr, nullptr);
 }
 
 template <typename R>
 struct OrderKernelsT {
-  VolLaunch<R> vol[4][2][2];     // [volume flux][ns][blend]
-  VolLaunch<R> vol_tma[4][2];    // bulk-copy-staged, no blending: [volume flux][ns]
+  VolLaunch<R> vol[4];           // [volume flux]
+  SmallLaunch<R> small[4][2];    // smaller meshes [volume flux][face terms too]
+  VolLaunch<R> vol_tma[4];       // bulk-copy-staged
   GradLaunch<R> grad;
   BlendLaunch<R> blend;
   VolLaunch<R> fv;               // subcell FV rate of blended elements
-  VolBatchLaunch<R> volb[4][2];  // [volume flux][ns]
+  VolBatchLaunch<R> volb[4];     // [volume flux]
   GradBatchLaunch<R> gradb;
   // half-size CTAs (epb_half elements each; 0 and null when EPB is 1)
   int epb, epb_half;
-  VolBatchLaunch<R> volb_half[4][2];
+  VolBatchLaunch<R> volb_half[4];
   GradBatchLaunch<R> gradb_half;
   // FP64 islands (Euler, blending; set in the FP64 units only)
   VolListLaunch<R> voll[4];      // [volume flux]

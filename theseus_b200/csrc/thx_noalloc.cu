@@ -193,7 +193,7 @@ extern "C" int thx_rhs_euler_noalloc(const thx_geometry *g, const thx_config *cf
                                                             : VOL_CENTRAL;
   VolLaunch<double> vol = nullptr;
 #define THX_NOALLOC_PICK(P, D, NN) \
-  if (dim == D && N == NN) vol = order_kernels_##P##_##D##_##NN().vol[vk][0][0];
+  if (dim == D && N == NN) vol = order_kernels_##P##_##D##_##NN().vol[vk];
   THX_FOR_ORDERS(THX_NOALLOC_PICK, 0, 2)
   THX_FOR_ORDERS(THX_NOALLOC_PICK, 0, 3)
 #undef THX_NOALLOC_PICK

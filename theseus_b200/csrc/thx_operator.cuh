@@ -133,6 +133,7 @@ struct thx_operator_s {
   float *sub32[3] = {nullptr, nullptr, nullptr}, *ops32 = nullptr, *D32 = nullptr;
   int *face_elem = nullptr, *face_lface = nullptr, *elem_face = nullptr;
   void *fstar = nullptr, *vflux = nullptr;  // face fluxes; NS physical viscous flux
+  void *vdiv = nullptr;      // NS: divergence of the viscous flux
   void *svars = nullptr;     // FP64 NS (ideal gas): entropy variables of every node
   int *face_order = nullptr; // interior faces sorted by their minus-side element
   double *alpha = nullptr, *eta = nullptr, *vinv = nullptr;
@@ -148,7 +149,12 @@ struct thx_operator_s {
   double *dtd = nullptr;   // device-side CFL time step (thx_rk3_steps_cfl)
   double *y = nullptr;
   float *yf = nullptr;
+  double *y2 = nullptr;    // second stage buffers of the fused small-mesh kernel
+  float *yf2 = nullptr;
   thx::Offsets off{};    // FP32 working-copy offsets (mixed mode)
+  int small = 0;           // smaller meshes: 1 small64 / small32 after the face kernel, 2 instead of it too
+  thx::SmallLaunch<double> small64 = nullptr;
+  thx::SmallLaunch<float> small32 = nullptr;
   thx::VolLaunch<double> vol64 = nullptr;
   thx::GradLaunch<double> grad64 = nullptr;
   thx::BlendLaunch<double> blend64 = nullptr;
