@@ -209,12 +209,14 @@ bool pick_order_kernels(thx_operator_s *h, int vk) {
       h->vol64 = reinterpret_cast<VolLaunch<double>>(tma ? k.vol_tma[vk] : k.vol[vk]); \
       h->small64 = reinterpret_cast<SmallLaunch<double>>(k.small[vk][h->small > 1]); \
       h->grad64 = reinterpret_cast<GradLaunch<double>>(k.grad);             \
+      h->gradl64 = reinterpret_cast<GradLineLaunch<double>>(k.grad_line);   \
       h->blend64 = reinterpret_cast<BlendLaunch<double>>(k.blend);          \
       h->fv64 = reinterpret_cast<VolLaunch<double>>(k.fv);                  \
     } else {                                                                \
       h->vol32 = reinterpret_cast<VolLaunch<float>>(tma ? k.vol_tma[vk] : k.vol[vk]); \
       h->small32 = reinterpret_cast<SmallLaunch<float>>(k.small[vk][h->small > 1]);  \
       h->grad32 = reinterpret_cast<GradLaunch<float>>(k.grad);              \
+      h->gradl32 = reinterpret_cast<GradLineLaunch<float>>(k.grad_line);    \
       h->blend32 = reinterpret_cast<BlendLaunch<float>>(k.blend);           \
       h->fv32 = reinterpret_cast<VolLaunch<float>>(k.fv);                   \
     }                                                                       \
@@ -351,6 +353,28 @@ void share_geometry(thx_operator_s *h, const thx_operator_s *d) {
   h->D64 = d->D64; h->D32 = d->D32;
   for (int k = 0; k < 3; ++k) { h->sub64[k] = d->sub64[k]; h->sub32[k] = d->sub32[k]; }
   h->vinv = d->vinv;
+}
+
+// Whether every element is a box along the axes, exactly: one metric per
+// element without off-diagonal entries, and face normals with no component
+// off the local face's axis.
+bool axis_aligned(const thx_geometry *g, const thx_operator_s *h) {
+  const int dim = h->dim;
+  if (h->lay.met_ns != 0 || h->lay.n_ps != 0) return false;
+  const int elems = h->lay.met_es == 0 ? 1 : h->ne;
+  for (int e = 0; e < elems; ++e)
+    for (int r = 0; r < dim; ++r)
+      for (int c = 0; c < dim; ++c)
+        if (r != c && g->metric[(size_t)e * h->nd * dim * dim + r * dim + c] != 0.0) return false;
+  for (int f = 0; f < h->nf; ++f)
+    for (int side = 0; side < 2; ++side)
+      for (int d = 0; d < dim; ++d)
+        if (d != g->face_lface[2 * f + side] >> 1 && g->face_normal[(size_t)f * h->nfp * dim + d] != 0.0) return false;
+  for (int b = 0; b < h->nbf; ++b)
+    for (int p = 0; p < h->nfp; ++p)
+      for (int d = 0; d < dim; ++d)
+        if (d != g->bdr_lface[b] >> 1 && g->bdr_normal[((size_t)b * h->nfp + p) * dim + d] != 0.0) return false;
+  return true;
 }
 
 int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
@@ -510,6 +534,9 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
   std::vector<double> x(N), w(N), D(N * N), Dh(N * N), Dh2(N * N);
   lgl_rule(N, x.data(), w.data());
   derivative_operators(N, x.data(), w.data(), D.data(), Dh.data(), Dh2.data());
+  h->hostD = D;
+  h->hostDhat = Dh;
+  h->aligned = h->ns && !h->lte && axis_aligned(g, h);
   if (!donor) {
     std::vector<double> ops(2 * N * N + N);
     std::memcpy(ops.data(), Dh2.data(), sizeof(double) * N * N);
@@ -643,6 +670,7 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
     ce = h->vol32(va, 0, 1);
     if (ce == cudaSuccess && h->small) ce = h->small32(va, FaceArgs<float>{}, 0, 0, 1);
     if (ce == cudaSuccess && h->ns) ce = h->grad32(ga, 0, 1);
+    if (ce == cudaSuccess && h->aligned) ce = h->gradl32(ga, nullptr, nullptr, 0, 1);
     if (ce == cudaSuccess && h->blend) ce = h->fv32(va, 0, 1);
     if (ce == cudaSuccess && h->islands) {
       VolArgs<double> v64{};
@@ -655,6 +683,7 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
     ce = h->vol64(va, 0, 1);
     if (ce == cudaSuccess && h->small) ce = h->small64(va, FaceArgs<double>{}, 0, 0, 1);
     if (ce == cudaSuccess && h->ns) ce = h->grad64(ga, 0, 1);
+    if (ce == cudaSuccess && h->aligned) ce = h->gradl64(ga, nullptr, nullptr, 0, 1);
     if (ce == cudaSuccess && h->blend && h->fv64) ce = h->fv64(va, 0, 1);
   }
   if (ce != cudaSuccess) { cudaGetLastError(); return THX_ERR_CUDA; }
@@ -689,6 +718,8 @@ EntropyLaunch<double> entk(thx_operator_s *h, double *) { return h->ent64; }
 EntropyLaunch<float> entk(thx_operator_s *h, float *) { return h->ent32; }
 GradLaunch<double> gradk(thx_operator_s *h, double *) { return h->grad64; }
 GradLaunch<float> gradk(thx_operator_s *h, float *) { return h->grad32; }
+GradLineLaunch<double> gradlk(thx_operator_s *h, double *) { return h->gradl64; }
+GradLineLaunch<float> gradlk(thx_operator_s *h, float *) { return h->gradl32; }
 BlendLaunch<double> blendk(thx_operator_s *h, double *) { return h->blend64; }
 VolLaunch<double> fvk(thx_operator_s *h, double *) { return h->fv64; }
 VolLaunch<float> fvk(thx_operator_s *h, float *) { return h->fv32; }
@@ -862,7 +893,12 @@ int run_rhs(thx_operator_s *h, const R *u, R *du, cudaStream_t s, int stage, dou
   if (h->svars &&
       entk(h, tag)(u, h->L, gas(h, tag), reinterpret_cast<R *>(h->svars), s) != cudaSuccess)
     return THX_ERR_CUDA;
-  if (h->ns && gradk(h, tag)(ga, s, 0) != cudaSuccess) return THX_ERR_CUDA;
+  // axis-aligned meshes of more than a few elements per SM: one thread per
+  // line (the node-parallel kernel has the shorter chains)
+  if (h->ns && (h->aligned && small == 0
+                    ? gradlk(h, tag)(ga, h->hostD.data(), h->hostDhat.data(), s, 0)
+                    : gradk(h, tag)(ga, s, 0)) != cudaSuccess)
+    return THX_ERR_CUDA;
   if (ev) cudaEventRecord(ev[2], s);
   if (small < 2 && facek(h, tag)(fa, s) != cudaSuccess) return THX_ERR_CUDA;
   if (isl && h->isl_face(fa64, h->isl_count + 1, s) != cudaSuccess) return THX_ERR_CUDA;

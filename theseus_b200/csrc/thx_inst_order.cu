@@ -35,6 +35,7 @@ THX_TYPE(THX_PREC) THX_NAME(THX_PREC, THX_DIM, THX_N)() {
 #else
   k.grad = &launch_grad<R, THX_DIM, THX_N>;     // FP32: evaluated in the kernel (cheaper)
 #endif
+  k.grad_line = &launch_grad_line<R, THX_DIM, THX_N>;
   k.blend = &launch_blend<R, THX_DIM, THX_N>;
   k.fv = &launch_fv<R, THX_DIM, THX_N>;
   k.gradb = &launch_grad_batched<R, THX_DIM, THX_N>;

@@ -1557,6 +1557,10 @@ __device__ __forceinline__ void grad_body_sv(const GradArgs<R> &a, const int blo
                                   e, active);
 }
 
+}  // namespace thx
+#include "thx_grad.cuh"
+namespace thx {
+
 template <typename R, int DIM, int N, bool LTE, bool SV = false>
 __global__ void __launch_bounds__(Shape<DIM, N>::THREADS) grad_kernel(const GradArgs<R> a) {
   grid_start();

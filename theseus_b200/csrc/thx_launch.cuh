@@ -163,6 +163,31 @@ cudaError_t launch_grad(const GradArgs<R> &a, cudaStream_t s, int prepare) {
   }
 }
 
+// Axis-aligned meshes: one thread per tensor line (ops: D and Dhat, on the
+// host).  FP64 reads the precomputed entropy variables.
+template <typename R>
+using GradLineLaunch = cudaError_t (*)(const GradArgs<R> &, const double *D, const double *Dhat, cudaStream_t, int);
+
+template <typename R, int DIM, int N>
+cudaError_t launch_grad_line(const GradArgs<R> &a, const double *D, const double *Dhat, cudaStream_t s, int prepare) {
+  constexpr int T = kLineThreads;
+  constexpr bool SV = !IsF32<R>::value;
+  using S = LineShape<DIM, N, T>;
+  constexpr size_t smem = GradLineSmem<R, DIM, N, T>::bytes();
+  if (prepare)
+    return cudaFuncSetAttribute(grad_line_kernel<R, DIM, N, T, SV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem);
+  if (a.ne <= 0) return cudaSuccess;
+  if (SV && !a.svars) return cudaErrorInvalidValue;
+  LineOps<R, N> m;
+  for (int i = 0; i < N * N; ++i) {
+    m.D[i] = (R)D[i];
+    m.Dhat[i] = (R)Dhat[i];
+  }
+  grad_line_kernel<R, DIM, N, T, SV><<<(a.ne + S::EPB - 1) / S::EPB, T, smem, s>>>(a, m);
+  return cudaGetLastError();
+}
+
 // Gradient from precomputed entropy variables (a.svars, entropy_kernel).
 template <typename R, int DIM, int N>
 cudaError_t launch_grad_sv(const GradArgs<R> &a, cudaStream_t s, int prepare) {
@@ -316,6 +341,7 @@ struct OrderKernelsT {
   SmallLaunch<R> small[4][2];    // smaller meshes [volume flux][face terms too]
   VolLaunch<R> vol_tma[4];       // bulk-copy-staged
   GradLaunch<R> grad;
+  GradLineLaunch<R> grad_line;   // axis-aligned meshes
   BlendLaunch<R> blend;
   VolLaunch<R> fv;               // subcell FV rate of blended elements
   VolBatchLaunch<R> volb[4];     // [volume flux]

@@ -155,6 +155,10 @@ struct thx_operator_s {
   int small = 0;           // smaller meshes: 1 small64 / small32 after the face kernel, 2 instead of it too
   thx::SmallLaunch<double> small64 = nullptr;
   thx::SmallLaunch<float> small32 = nullptr;
+  bool aligned = false;    // elements are boxes along the axes (exactly)
+  std::vector<double> hostD, hostDhat;  // derivative operators
+  thx::GradLineLaunch<double> gradl64 = nullptr;
+  thx::GradLineLaunch<float> gradl32 = nullptr;
   thx::VolLaunch<double> vol64 = nullptr;
   thx::GradLaunch<double> grad64 = nullptr;
   thx::BlendLaunch<double> blend64 = nullptr;
