@@ -26,23 +26,29 @@ struct GradLineSmem {
   using S = LineShape<DIM, N, T>;
   static constexpr int FIELDS = DIM * S::NEQ;  // entropy variables, then the other directions' gradients
   static constexpr size_t bytes() {
-    return sizeof(R) * (size_t)FIELDS * S::FS + sizeof(int) * S::EPB * 2 * DIM;
+    return sizeof(R) * (size_t)FIELDS * S::FS + sizeof(int) * 3 * S::EPB * 2 * DIM;
   }
 };
 
-// Entropy variables at node i of the state (SV: stored; otherwise evaluated
-// from the working state, or from the FP64 state narrowed as grad_body does).
+// What the entropy variables at node i are formed from: themselves (SV:
+// stored), or the working state, narrowed from the FP64 state as grad_body
+// does where that is given.
 template <typename R, int DIM, bool SV>
-__device__ __forceinline__ void entropy_at(const GradArgs<R> &a, const long long L, const long long i, R *w) {
-  constexpr int NEQ = DIM + 2;
+__device__ __forceinline__ void entropy_load(const GradArgs<R> &a, const long long L, const long long i, R *x) {
+#pragma unroll
+  for (int k = 0; k < DIM + 2; ++k) {
+    if (SV) x[k] = a.svars[k * L + i];
+    else x[k] = a.u64 ? (R)(a.u64[k * L + i] - a.off[k]) : a.u[k * L + i];
+  }
+}
+template <typename R, int DIM, bool SV>
+__device__ __forceinline__ void entropy_from(const GradArgs<R> &a, const R *x, R *w) {
   if constexpr (SV) {
 #pragma unroll
-    for (int k = 0; k < NEQ; ++k) w[k] = a.svars[k * L + i];
+    for (int k = 0; k < DIM + 2; ++k) w[k] = x[k];
   } else {
-    R raw[NEQ], q[NEQ];
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k) raw[k] = a.u64 ? (R)(a.u64[k * L + i] - a.off[k]) : a.u[k * L + i];
-    reconstruct<R, DIM>(a.gas, raw, q);
+    R q[DIM + 2];
+    reconstruct<R, DIM>(a.gas, x, q);
     entropy_vars<R, DIM>(a.gas, q, w);
   }
 }
@@ -61,31 +67,46 @@ grad_line_kernel(const GradArgs<R> a, const LineOps<R, N> m) {
   R *sS = reinterpret_cast<R *>(smem_raw);                     // [NEQ][EPB][NDP] entropy variables
   R *sG = sS + NEQ * FS;                                       // [DIM-1][NEQ][EPB][NDP] gradients
   int *sF = reinterpret_cast<int *>(sS + M::FIELDS * FS);      // [EPB][2*DIM] elem_face
+  int *sNE = sF + EPB * 2 * DIM, *sNL = sNE + EPB * 2 * DIM;   // the neighbours' elements and local faces
   const int tid = threadIdx.x;
   const int e0 = blockIdx.x * EPB;
   const long long L = (long long)a.ne * ND;
   const int nodes = min(EPB, a.ne - e0) * ND;
-  for (int i = tid; i < nodes / ND * 2 * DIM; i += T) sF[i] = a.elem_face[(long long)e0 * 2 * DIM + i];
+  // every load of the thread's nodes is issued before the first use
+  constexpr int IT = (EPB * ND + T - 1) / T;
+  R xn[IT][NEQ];
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int i = tid + it * T;
+    if (i < nodes) entropy_load<R, DIM, SV>(a, L, (long long)e0 * ND + i, xn[it]);
+  }
+  for (int i = tid; i < nodes / ND * 2 * DIM; i += T) {
+    const int fs = a.elem_face[(long long)e0 * 2 * DIM + i];
+    const bool in = fs >= 0 && !(a.bw && (fs >> 1) >= a.nf_int);
+    sF[i] = fs;
+    sNE[i] = in ? a.face_elem[2 * (fs >> 1) + 1 - (fs & 1)] : 0;
+    sNL[i] = in ? a.face_lface[2 * (fs >> 1) + 1 - (fs & 1)] : 0;
+  }
   bool bad = false;
 #pragma unroll
-  for (int it = 0; it < (EPB * ND + T - 1) / T; ++it) {
+  for (int it = 0; it < IT; ++it) {
     const int i = tid + it * T;
     if (i >= nodes) continue;
-    const long long gi = (long long)e0 * ND + i;
     R w[NEQ];
     if constexpr (IsF32<R>::value) {
       if (a.u64) {
         // the working copy of the node for the kernels that follow, and the
         // positivity of its FP64 state
+        const long long gi = (long long)e0 * ND + i;
         double d[NEQ];
 #pragma unroll
         for (int k = 0; k < NEQ; ++k) d[k] = a.u64[k * L + gi];
 #pragma unroll
-        for (int k = 0; k < NEQ; ++k) a.yf[k * L + gi] = (float)(R)(d[k] - a.off[k]);
+        for (int k = 0; k < NEQ; ++k) a.yf[k * L + gi] = (float)xn[it][k];
         if (!fp64_state_positive<DIM>(d, (double)a.gas.gm1)) bad = true;
       }
     }
-    entropy_at<R, DIM, SV>(a, L, gi, w);
+    entropy_from<R, DIM, SV>(a, xn[it], w);
     const int pn = i + (N % 2 ? 0 : i / N);
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) sS[k * FS + pn] = w[k];
@@ -98,6 +119,21 @@ grad_line_kernel(const GradArgs<R> a, const LineOps<R, N> m) {
   const bool active = el < EPB && e < a.ne;
   const R *met = a.met + (long long)e * a.met_es;
   const R *jac = a.jac + (long long)e * a.jac_es;
+  // the neighbours' traces, lift weights and normals at the ends of the
+  // thread's lines: every gather is issued before the first derivative
+  R so[DIM][2][NEQ], lw[DIM][2], ln[DIM][2];
+  if (active) {
+#pragma unroll
+    for (int dir = 0; dir < DIM; ++dir)
+#pragma unroll
+      for (int hi = 0; hi < 2; ++hi) {
+        const int lf = el * 2 * DIM + 2 * dir + hi, fs = sF[lf], f = fs >> 1;
+        if (fs < 0 || (a.bw && f >= a.nf_int)) continue;
+        entropy_load<R, DIM, SV>(a, L, (long long)sNE[lf] * ND + trace_node<DIM>(N, sNL[lf], line), so[dir][hi]);
+        lw[dir][hi] = ((fs & 1) == 0 ? a.wm : a.wp)[(long long)f * a.w_fs + (long long)line * a.w_ps];
+        ln[dir][hi] = a.normal[((long long)f * a.n_fs + (long long)line * a.n_ps) * DIM + dir];
+      }
+  }
   // gradient along `dir` of the thread's line: invJ * (D-derivative * metric)
   // plus the lift of the end nodes' faces
   auto gradient = [&](auto dirc, R *dst) {
@@ -133,17 +169,13 @@ grad_line_kernel(const GradArgs<R> a, const LineOps<R, N> m) {
         }
       }
       // interior face: w * 0.5 (S+ - S-) n
-      const int eo = a.face_elem[2 * f + 1 - side];
-      const int no = trace_node<DIM>(N, a.face_lface[2 * f + 1 - side], line);
-      R so[NEQ];
-      entropy_at<R, DIM, SV>(a, L, (long long)eo * ND + no, so);
-      const R w = (side == 0 ? a.wm : a.wp)[(long long)f * a.w_fs + (long long)line * a.w_ps];
-      const R n = a.normal[((long long)f * a.n_fs + (long long)line * a.n_ps) * DIM + dir];
+      R st[NEQ];
+      entropy_from<R, DIM, SV>(a, so[dir][hi], st);
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) {
         const R sown = sS[k * FS + own];
-        const R jump = side == 0 ? R(0.5) * (so[k] - sown) : R(0.5) * (sown - so[k]);
-        lift[hi][k] += w * (jump * n);
+        const R jump = side == 0 ? R(0.5) * (st[k] - sown) : R(0.5) * (sown - st[k]);
+        lift[hi][k] += lw[dir][hi] * (jump * ln[dir][hi]);
       }
     }
     const R ar = met[dir * DIM + dir];
@@ -151,7 +183,9 @@ grad_line_kernel(const GradArgs<R> a, const LineOps<R, N> m) {
 #pragma unroll
     for (int i = 0; i < N; ++i)
       ij[i] = i > 0 && a.jac_ns == 0 ? ij[0] : R(1) / jac[(long long)line_node<DIM, N>(dir, line, i) * a.jac_ns];
-#pragma unroll
+    // rolled over the variables: unrolled, the kernel outgrows the
+    // instruction cache
+#pragma unroll 1
     for (int k = 0; k < NEQ; ++k) {
       R s[N];
 #pragma unroll
@@ -162,12 +196,15 @@ grad_line_kernel(const GradArgs<R> a, const LineOps<R, N> m) {
 #pragma unroll
         for (int l = 0; l < N; ++l) g += s[l] * m.D[i * N + l];
         g = g * ar;
-        g = ij[i] * g;
-        if (i == 0 && lifted[0]) g += lift[0][k];
-        if (i == N - 1 && lifted[1]) g += lift[1][k];
-        dst[k * FS + base + i * stride] = g;
+        dst[k * FS + base + i * stride] = ij[i] * g;
       }
     }
+#pragma unroll
+    for (int hi = 0; hi < 2; ++hi)
+      if (lifted[hi]) {
+#pragma unroll
+        for (int k = 0; k < NEQ; ++k) dst[k * FS + base + (hi ? N - 1 : 0) * stride] += lift[hi][k];
+      }
   };
   if (active) {
     gradient(std::integral_constant<int, 0>{}, sG);
@@ -186,17 +223,24 @@ grad_line_kernel(const GradArgs<R> a, const LineOps<R, N> m) {
     R row[DIM];
 #pragma unroll
     for (int d = 0; d < DIM; ++d) row[d] = met[d * DIM + d];
+    // the next node's state is loaded while this one's flux is formed
+    R next[NEQ];
+    auto fetch = [&](int i) {
+      const long long gi = (long long)e * ND + line + i * NL;
+#pragma unroll
+      for (int k = 0; k < NEQ; ++k) {
+        if (!SV && a.u64) next[k] = (R)(a.u64[k * L + gi] - a.off[k]);
+        else next[k] = a.u[k * L + gi];
+      }
+    };
+    fetch(0);
 #pragma unroll 1
     for (int i = 0; i < N; ++i) {
       const int s = base + i * stride, n = line + i * NL;
       const long long gi = (long long)e * ND + n;
-      R raw[NEQ], q[NEQ], g[DIM][NEQ];
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) {
-        if (!SV && a.u64) raw[k] = (R)(a.u64[k * L + gi] - a.off[k]);
-        else raw[k] = a.u[k * L + gi];
-      }
-      reconstruct<R, DIM>(a.gas, raw, q);
+      R q[NEQ], g[DIM][NEQ];
+      reconstruct<R, DIM>(a.gas, next, q);
+      if (i + 1 < N) fetch(i + 1);
       const NodeGas<R, DIM> ng = node_gas<R, DIM>(a.gas, q);
 #pragma unroll
       for (int cc = 0; cc < DIM; ++cc) {
@@ -255,7 +299,7 @@ grad_line_kernel(const GradArgs<R> a, const LineOps<R, N> m) {
     int base, stride;
     line_base<DIM, N, S::LS>(dir, line, base, stride);
     base += el * S::NDP;
-#pragma unroll
+#pragma unroll 1
     for (int k = 0; k < NV; ++k) {
       R f[N];
 #pragma unroll

@@ -1046,7 +1046,8 @@ __global__ void __launch_bounds__(256) entropy_kernel(const R *__restrict__ u, l
 #pragma unroll
   for (int k = 0; k < NEQ; ++k) raw[k] = u[k * L + i];
   reconstruct<R, DIM>(gas, raw, q);
-  entropy_vars<R, DIM>(gas, q, w);
+  if constexpr (IsF32<R>::value) entropy_vars<R, DIM>(gas, q, w);
+  else entropy_vars_shared<DIM>(gas, q, w);
 #pragma unroll
   for (int k = 0; k < NEQ; ++k) sv[k * L + i] = w[k];
 }

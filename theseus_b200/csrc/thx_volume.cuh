@@ -263,6 +263,30 @@ __device__ __forceinline__ void line_base(int dir, int line, int &base, int &str
   }
 }
 
+// entropy_vars (thx_device.cuh) with the seven quotients formed from two
+// reciprocals where density and pressure are in their range: the same
+// operations in the same order.
+template <int DIM>
+__device__ __forceinline__ void entropy_vars_shared(const GasT<double> &g, const double *q, double *w) {
+  const double rho = q[0];
+  double m2 = 0.0;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) m2 += q[1 + d] * q[1 + d];
+  const double yr = rcp_refined(rho);
+  const double ke = div_by(0.5 * m2, rho, yr);
+  const double p = g.gm1 * (q[DIM + 1] - ke);
+  if (!in_fast_range(rho) || !in_fast_range(p)) {
+    entropy_vars<double, DIM>(g, q, w);
+    return;
+  }
+  const double s = rlog(p) - g.gamma * rlog(rho);
+  const double beta = div_by(rho, p, rcp_refined(p));
+  w[0] = div_by(g.gamma - s, g.gamma - 1.0, g.inv_gm1) - beta * div_by(ke, rho, yr);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) w[1 + d] = beta * div_by(q[1 + d], rho, yr);
+  w[DIM + 1] = -beta;
+}
+
 // Lift weight of face point fp of an elem_face entry; zero (and false) without
 // an interior face.
 template <typename R, int DIM, int NFP>
