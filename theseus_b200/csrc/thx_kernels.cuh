@@ -539,6 +539,10 @@ __device__ __forceinline__ void volume_body(const VolArgs<R> &a, const int block
   }
 }
 
+template <int DIM, int SURF>
+__device__ __forceinline__ bool try_surface_flux_shared(const GasT<double> &g, const int kind, const double *qm,
+                                                        const double *qp, const double *n, double *F);
+
 // Subcell finite-volume rate of the blended elements (include/DGSEMIntegrator.hpp:338-483):
 // along every tensor line, first-order fluxes F_j between neighbouring
 // subcells j, j+1 with the run-time FV face flux; node i of the line gets
@@ -591,23 +595,28 @@ __device__ __forceinline__ void fv_body(const VolArgs<R> &a, const int block) {
     const int fel = t / FACES;
     const int r = t - fel * FACES;
     const int dir = r / (NL * (N - 1));
-    const int r2 = r - dir * (NL * (N - 1));
-    const int line = r2 / (N - 1), j = r2 - line * (N - 1);
+    const int rd = r - dir * (NL * (N - 1));
+    const int line = rd / (N - 1), j = rd - line * (N - 1);
     const int fe = e0 + fel;
     if (fe >= a.ne || !(a.alpha[fe] > 1e-16)) continue;
     const int id1 = line_node<DIM, N>(dir, line, j), id2 = line_node<DIM, N>(dir, line, j + 1);
-    R raw[NEQ], fn[NEQ], nrm[DIM];
-    FState<R, DIM> s1, s2;
+    R r1[NEQ], r2[NEQ], fn[NEQ], nrm[DIM];
 #pragma unroll
-    for (int k = 0; k < NEQ; ++k) raw[k] = sQ[(fel * NEQ + k) * ND + id1];
-    make_fstate<R, DIM>(a.gas, raw, s1);
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k) raw[k] = sQ[(fel * NEQ + k) * ND + id2];
-    make_fstate<R, DIM>(a.gas, raw, s2);
+    for (int k = 0; k < NEQ; ++k) {
+      r1[k] = sQ[(fel * NEQ + k) * ND + id1];
+      r2[k] = sQ[(fel * NEQ + k) * ND + id2];
+    }
     const R *sub = a.sub[dir] + (long long)fe * a.sub_es[dir];
 #pragma unroll
     for (int d = 0; d < DIM; ++d) nrm[d] = sub[id2 * DIM + d];
-    surface_flux_rt<R, DIM>(a.fv_flux, a.gas, s1, s2, nrm, fn);
+    bool done = false;
+    if constexpr (!IsF32<R>::value) done = try_surface_flux_shared<DIM, -1>(a.gas, a.fv_flux, r1, r2, nrm, fn);
+    if (!done) {
+      FState<R, DIM> s1, s2;
+      make_fstate<R, DIM>(a.gas, r1, s1);
+      make_fstate<R, DIM>(a.gas, r2, s2);
+      surface_flux_rt<R, DIM>(a.fv_flux, a.gas, s1, s2, nrm, fn);
+    }
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) sF[((long long)fel * FACES + r) * NEQ + k] = fn[k];
   }
@@ -841,6 +850,10 @@ struct FaceArgs {
   const int *order;
 };
 
+}  // namespace thx
+#include "thx_face.cuh"
+namespace thx {
+
 // Flux F* of point fp of face f (minus to plus side).  SURF < 0: the surface
 // flux is chosen at run time (kind).
 template <typename R, int DIM, int SURF, bool NS>
@@ -868,11 +881,15 @@ __device__ __forceinline__ void face_point_flux(const FaceArgs<R> &a, const int 
     lte_ec_flux<DIM, true>(a.gas.lte, qm, qp, sm, sp, lte_face_jet(a.gas.lte, sm),
                            lte_face_jet(a.gas.lte, sp), nrm, nrm, F);
   } else {
-    FState<R, DIM> A, B;
-    make_fstate<R, DIM>(a.gas, qm, A);
-    make_fstate<R, DIM>(a.gas, qp, B);
-    if constexpr (SURF < 0) surface_flux_rt<R, DIM>(kind, a.gas, A, B, nrm, F);
-    else surface_flux<R, DIM, SURF>(a.gas, A, B, nrm, F);
+    bool done = false;
+    if constexpr (!IsF32<R>::value) done = try_surface_flux_shared<DIM, SURF>(a.gas, kind, qm, qp, nrm, F);
+    if (!done) {
+      FState<R, DIM> A, B;
+      make_fstate<R, DIM>(a.gas, qm, A);
+      make_fstate<R, DIM>(a.gas, qp, B);
+      if constexpr (SURF < 0) surface_flux_rt<R, DIM>(kind, a.gas, A, B, nrm, F);
+      else surface_flux<R, DIM, SURF>(a.gas, A, B, nrm, F);
+    }
   }
   if (NS) {
     // include/DGSEMIntegrator.hpp:261-316: F* -= n . avg(F_v), with the physical
