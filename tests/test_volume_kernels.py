@@ -14,11 +14,11 @@ from _helpers import box, oracle_mesh, random_geometry, rel_l2, smooth_state, to
 pytestmark = pytest.mark.gpu
 
 TOL = 1e-12
-# CTAs of the small-mesh kernel: within two per SM, within five, beyond
+# meshes that take the small-mesh kernel with the face terms, without, and the line kernel
 SIZES = {(2, 2): ((9, 7), (97, 95), (147, 149)), (2, 3): ((9, 7), (65, 63), (97, 95)),
-         (2, 4): ((9, 7), (41, 39), (63, 61)), (2, 5): ((9, 7), (31, 29), (43, 41)),
-         (3, 2): ((3, 4, 5), (14, 15, 13), (19, 17, 18)), (3, 3): ((3, 4, 5), (8, 9, 7), (10, 11, 9)),
-         (3, 4): ((3, 4, 5), (8, 7, 9), (10, 9, 11)), (3, 5): ((3, 4, 5), (7, 8, 9), (9, 10, 11))}
+         (2, 4): ((9, 7), (41, 39), (73, 71)), (2, 5): ((9, 7), (31, 29), (61, 59)),
+         (3, 2): ((3, 4, 5), (14, 15, 13), (19, 17, 18)), (3, 3): ((3, 4, 5), (8, 9, 7), (13, 12, 13)),
+         (3, 4): ((3, 4, 5), (8, 7, 9), (10, 9, 11)), (3, 5): ((3, 4, 5), (7, 7, 8), (9, 10, 11))}
 
 
 def rough_state(m, seed, ratio):

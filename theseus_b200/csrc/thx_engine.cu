@@ -199,7 +199,10 @@ class Engine final : public EngineBase {
       cudaStreamSynchronize(setup_);
       cudaStreamDestroy(setup_);
     }
-    for (Bounce &b : bounce_) cudaFreeHost(b.ptr);
+    for (Bounce &b : bounce_) {
+      if (b.stream) cudaStreamDestroy(b.stream);
+      cudaFreeHost(b.ptr);
+    }
     if (pool_) cudaMemPoolDestroy(pool_);
   }
 
@@ -337,24 +340,27 @@ class Engine final : public EngineBase {
   int upload_working_copy(thx_operator_s *h, const double *u0) {
     const long long L = h->L;
     const int neq = h->neq, dim = h->dim;
-    thread_local std::vector<float> wf;
-    wf.resize((size_t)L * neq);
-    for (int k = 0; k < neq; ++k) {
-      const double o = h->off.v[k];
-      const double *src = u0 + (size_t)k * L;
-      float *dst = wf.data() + (size_t)k * L;
-      for (long long i = 0; i < L; ++i) dst[i] = (float)(src[i] - o);
-    }
-    bool bad = false;
+    // straight into the pinned ring, without a buffer of its own
+    int st = ring_.fill(h->yf, (size_t)L * neq * sizeof(float), setup_, [&](void *to) {
+      for (int k = 0; k < neq; ++k) {
+        const double o = h->off.v[k];
+        const double *__restrict__ src = u0 + (size_t)k * L;
+        float *__restrict__ dst = (float *)to + (size_t)k * L;
+        for (long long i = 0; i < L; ++i) dst[i] = (float)(src[i] - o);
+      }
+    });
+    // no early exit: the loop stays vectorised
+    int bad = 0;
     const double gm1 = h->g64.gm1;
-    for (long long i = 0; i < L && !bad; ++i) {
-      double m2 = 0.0;
-      for (int d = 0; d < dim; ++d) m2 += u0[(size_t)(1 + d) * L + i] * u0[(size_t)(1 + d) * L + i];
-      const double rho = u0[i];
-      const double p = gm1 * (u0[(size_t)(dim + 1) * L + i] - 0.5 * m2 / rho);
-      bad = !(rho > 0.0 && p > 0.0);
+    const double *rho = u0, *mx = u0 + L, *my = u0 + 2 * L, *mz = dim == 3 ? u0 + 3 * L : nullptr;
+    const double *en = u0 + (size_t)(dim + 1) * L;
+    for (long long i = 0; i < L; ++i) {
+      double m2 = 0.0 + mx[i] * mx[i];
+      m2 += my[i] * my[i];
+      if (mz) m2 += mz[i] * mz[i];
+      const double p = gm1 * (en[i] - 0.5 * m2 / rho[i]);
+      bad |= !(rho[i] > 0.0) | !(p > 0.0);
     }
-    int st = ring_.copy(h->yf, wf.data(), wf.size() * sizeof(float), setup_);
     if (!st && bad) {
       static const unsigned flag = STATUS_NONPOSITIVE;
       st = ring_.copy(h->status, &flag, sizeof(flag), setup_);
@@ -408,13 +414,15 @@ class Engine final : public EngineBase {
     // driver's slow path)
     const size_t bytes = n * sizeof(double);
     Bounce b = take_bounce(bytes);
-    cudaStream_t fs = nullptr;
-    cudaError_t e = b.ptr ? cudaStreamCreateWithFlags(&fs, cudaStreamNonBlocking) : cudaErrorMemoryAllocation;
+    cudaStream_t fs = b.stream;
+    cudaError_t e = !b.ptr ? cudaErrorMemoryAllocation
+                    : fs   ? cudaSuccess
+                           : cudaStreamCreateWithFlags(&fs, cudaStreamNonBlocking);
+    b.stream = e == cudaSuccess ? fs : nullptr;
     if (e == cudaSuccess) e = cudaStreamWaitEvent(fs, c->done, 0);
     if (e == cudaSuccess) e = cudaMemcpyAsync(b.ptr, c->u, bytes, cudaMemcpyDeviceToHost, fs);
     if (e == cudaSuccess) e = cudaStreamSynchronize(fs);
     if (e == cudaSuccess) std::memcpy(u_host, b.ptr, bytes);
-    if (fs) cudaStreamDestroy(fs);
     give_bounce(b);
     std::lock_guard<std::mutex> lock(mu_);
     t_fetch_ += now() - t0;
@@ -480,6 +488,7 @@ class Engine final : public EngineBase {
   using Key = std::tuple<int, int, bool>;
 
   struct Bounce {
+    cudaStream_t stream = nullptr;  // the copies' stream, kept with the buffer
     unsigned char *ptr = nullptr;
     size_t size = 0;
   };

@@ -45,7 +45,14 @@ THX_TYPE(THX_PREC) THX_NAME(THX_PREC, THX_DIM, THX_N)() {
   k.gradb_half = nullptr;
   if constexpr (half_epb<THX_DIM, THX_N>() > 0) {
     constexpr int H = half_epb<THX_DIM, THX_N>();
+    // FP64: the line and the pair kernel give the same bits.  FP32 may contract
+    // multiply-adds differently in the two, and a case's result must not depend
+    // on what the tuner finds for the cases beside it.
+#if THX_PREC == 0
+#define THX_SETH(V) k.volb_half[V] = &launch_volume_batched_pairs<R, THX_DIM, THX_N, V, H>;
+#else
 #define THX_SETH(V) k.volb_half[V] = &launch_volume_batched<R, THX_DIM, THX_N, V, H>;
+#endif
     THX_SETH(VOL_CHANDRASHEKAR)
     THX_SETH(VOL_RANOCHA)
     THX_SETH(VOL_PIROZZOLI)

@@ -2055,6 +2055,24 @@ volume_batched(const VolArgs<R> *__restrict__ args, const BatchWork *__restrict_
   }
 }
 
+// Half-size work items: one thread per pair (small_body), for groups whose
+// lines are too few to fill the chip.
+template <typename R, int DIM, int N, int VOL, int EPBX>
+__global__ void __launch_bounds__(kSmallThreads, (small_min_blocks<R, false>()))
+volume_batched_pairs(const VolArgs<R> *__restrict__ args, const BatchWork *__restrict__ work,
+                     const int *__restrict__ nwork) {
+  __shared__ __align__(16) unsigned char sa[sizeof(VolArgs<R>)];
+  const int n = *nwork;
+  for (int w = blockIdx.x; w < n; w += gridDim.x) {
+    __syncthreads();  // the previous item's shared memory is free
+    const BatchWork it = work[w];
+    stage_record(sa, &args[it.item]);
+    __syncthreads();
+    small_body<R, DIM, N, VOL, false, false>(*reinterpret_cast<const VolArgs<R> *>(sa), FaceArgs<R>{}, 0, EPBX,
+                                             it.block * EPBX);
+  }
+}
+
 template <typename R, int DIM, int N, int EPBX = 0>
 __global__ void __launch_bounds__(Shape<DIM, N, EPBX>::THREADS)
 grad_batched(const GradArgs<R> *__restrict__ args, const BatchWork *__restrict__ work,

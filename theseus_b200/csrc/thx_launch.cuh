@@ -98,12 +98,12 @@ using SmallLaunch = cudaError_t (*)(const VolArgs<R> &, const FaceArgs<R> &, int
 template <typename R, int DIM, int N, int VOL, bool FACES>
 cudaError_t launch_volume_small(const VolArgs<R> &a, const FaceArgs<R> &fa, int surf, cudaStream_t s, int prepare) {
   using M = SmallSmem<R, DIM, N, VOL, FACES>;
-  const int epb = small_epb(DIM, N, a.ne);
-  static_assert(M::bytes(small_epb(DIM, N, 1 << 30)) <= 200 * 1024, "shared memory");
+  const int epb = small_epb(DIM, N, a.ne, FACES);
+  static_assert(M::bytes(small_epb(DIM, N, 1 << 30, FACES)) <= 200 * 1024, "shared memory");
   if (prepare)
     return cudaFuncSetAttribute(volume_small_kernel<R, DIM, N, VOL, FACES>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)M::bytes(small_epb(DIM, N, 1 << 30)));
+                                (int)M::bytes(small_epb(DIM, N, 1 << 30, FACES)));
   if (a.ne <= 0) return cudaSuccess;
   return launch_early(volume_small_kernel<R, DIM, N, VOL, FACES>, (a.ne + epb - 1) / epb, kSmallThreads, M::bytes(epb), s, a, fa, surf, epb);
 }
@@ -231,6 +231,18 @@ cudaError_t launch_volume_batched(const VolArgs<R> *args, const BatchWork *work,
   // the tuned grid counts CTAs of Shape's threads; this kernel's are smaller
   constexpr int scale = Shape<DIM, N, EPBX>::THREADS / T;
   volume_batched<R, DIM, N, VOL, EPBX><<<grid * scale, T, smem, s>>>(args, work, nwork);
+  return cudaGetLastError();
+}
+
+template <typename R, int DIM, int N, int VOL, int EPBX>
+cudaError_t launch_volume_batched_pairs(const VolArgs<R> *args, const BatchWork *work, const int *nwork,
+                                        int grid, cudaStream_t s, int prepare) {
+  constexpr size_t smem = SmallSmem<R, DIM, N, VOL, false>::bytes(EPBX);
+  if (prepare)
+    return cudaFuncSetAttribute(volume_batched_pairs<R, DIM, N, VOL, EPBX>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (grid <= 0) return cudaSuccess;
+  volume_batched_pairs<R, DIM, N, VOL, EPBX><<<grid, kSmallThreads, smem, s>>>(args, work, nwork);
   return cudaGetLastError();
 }
 

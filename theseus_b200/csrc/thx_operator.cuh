@@ -55,12 +55,23 @@ class HostRing {
   // host -> device copy of `bytes` on stream s through the ring (copies of
   // more than half the ring go directly)
   int copy(void *dst, const void *src, size_t bytes, cudaStream_t s) {
-    std::lock_guard<std::mutex> lock(mu_);
-    const size_t need = (bytes + 255) & ~size_t(255);
-    if (!buf_ || need > space_.capacity() / 2) {
+    if (!fits(bytes)) {
       const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
       return e == cudaSuccess ? THX_OK : cuda_failed(e, "cudaMemcpyAsync(upload)");
     }
+    return fill(dst, bytes, s, [&](void *to) { std::memcpy(to, src, bytes); });
+  }
+  // the same with the bytes written by write(to), in the ring where they fit
+  template <typename F>
+  int fill(void *dst, size_t bytes, cudaStream_t s, F &&write) {
+    if (!fits(bytes)) {
+      std::vector<unsigned char> own(bytes);
+      write(own.data());
+      const cudaError_t e = cudaMemcpyAsync(dst, own.data(), bytes, cudaMemcpyHostToDevice, s);
+      return e == cudaSuccess ? THX_OK : cuda_failed(e, "cudaMemcpyAsync(upload)");
+    }
+    std::lock_guard<std::mutex> lock(mu_);
+    const size_t need = (bytes + 255) & ~size_t(255);
     size_t off;
     const auto t0 = std::chrono::steady_clock::now();
     while (!space_.place(need, &off)) {  // wait for the oldest copy
@@ -71,7 +82,7 @@ class HostRing {
       space_.pop();
     }
     const auto t1 = std::chrono::steady_clock::now();
-    std::memcpy(buf_ + off, src, bytes);
+    write(buf_ + off);
     const auto t2 = std::chrono::steady_clock::now();
     wait_s_ += std::chrono::duration<double>(t1 - t0).count();
     copy_s_ += std::chrono::duration<double>(t2 - t1).count();
@@ -103,6 +114,7 @@ class HostRing {
   }
 
  private:
+  bool fits(size_t bytes) const { return buf_ && ((bytes + 255) & ~size_t(255)) <= space_.capacity() / 2; }
   std::mutex mu_;
   double wait_s_ = 0.0, copy_s_ = 0.0;
   unsigned char *buf_ = nullptr;

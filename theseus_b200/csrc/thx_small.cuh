@@ -15,26 +15,30 @@ namespace thx {
 constexpr int kSmallThreads = 256;
 constexpr int kSmallSMs = 148;
 
-// Elements per CTA: spread over the SMs, up to about two pairs per thread.
-__host__ constexpr int small_epb(int dim, int N, int ne) {
-  const int pairs = dim * (dim == 2 ? N : N * N) * (N * (N - 1) / 2);
-  const int busy = 2 * kSmallThreads / pairs > 0 ? 2 * kSmallThreads / pairs : 1;
-  const int spread = (ne + kSmallSMs - 1) / kSmallSMs;
-  return spread < 1 ? 1 : spread < busy ? spread : busy;
+// Elements per CTA.  With the face terms: spread over the SMs, up to about two
+// pairs per thread.  Without: over three CTAs per SM (all resident), up to a
+// node per thread.
+__host__ constexpr int small_epb(int dim, int N, int ne, bool faces) {
+  const int nd = dim == 2 ? N * N : N * N * N;
+  const int pairs = dim * (nd / N) * (N * (N - 1) / 2);
+  const int most = faces ? 2 * kSmallThreads / pairs : kSmallThreads / nd;
+  const int ctas = faces ? kSmallSMs : 3 * kSmallSMs;
+  const int spread = (ne + ctas - 1) / ctas;
+  const int epb = spread < most ? spread : most;
+  return epb > 1 ? epb : 1;
 }
 
 // Which volume kernel a mesh takes: 2 this one with the face terms, 1 this one
 // after the face kernel, 0 the line kernel after the face kernel.  The first
-// while its CTAs are resident at once (two per SM, by its registers): RK3
-// stage of the 2-D Euler vortex, FP64, against the line kernel, 32^2 p=3 9.8
-// against 21.6 us, 48^2 10.3 / 22.0, 32^2 p=5 18.5 / 34.2.  The second up to
-// five CTAs per SM, where the line kernel's threads are too few to hide its
-// longer chains: 64^2 p=3 15.8 / 22.2 (16.4 for the first), 3-D 9^3 p=3 22.7 /
-// 28.7, 9^3 p=4 32.6 / 40.3.  Beyond, the line kernel's fewer instructions win:
-// 96^2 p=3 22.6 against 24.1 us, 12^3 p=4 54.0 / 60.7, 96^2 p=5 40.5 / 76.8.
+// two while their CTAs are resident at once (two and three per SM, by their
+// registers); beyond, the line kernel's fewer instructions outweigh its longer
+// chains.  RK3 stage of the 2-D Euler vortex, FP64, first / second / line
+// kernel: 32^2 p=3 9.8 / 13.7 / 21.6 us, 48^2 10.3 / 14.4 / 22.0, 64^2 16.4 /
+// 15.8 / 22.2, 96^2 28.7 / 24.1 / 22.6, 128^2 44.3 / 32.8 / 28.5; 3-D p=3 5^3
+// 10.3 / 16.4 / 28.7, 7^3 18.5 / 16.4 / 28.7, 16^3 110 / 85 / 51.
 __host__ constexpr int small_mesh(int dim, int N, int ne) {
-  const int epb = small_epb(dim, N, ne), ctas = (ne + epb - 1) / epb;
-  return ctas <= 2 * kSmallSMs ? 2 : ctas <= 5 * kSmallSMs ? 1 : 0;
+  const int e2 = small_epb(dim, N, ne, true), e1 = small_epb(dim, N, ne, false);
+  return (ne + e2 - 1) / e2 <= 2 * kSmallSMs ? 2 : (ne + e1 - 1) / e1 <= 3 * kSmallSMs ? 1 : 0;
 }
 
 template <typename R, int DIM, int N, int VOL, bool FACES>
@@ -52,16 +56,17 @@ struct SmallSmem {
   }
 };
 
-// FACES: the kernel evaluates the face fluxes itself; otherwise the face kernel
-// has stored them.
-template <typename R, int DIM, int N, int VOL, bool FACES>
-__global__ void __launch_bounds__(kSmallThreads, FACES ? 2 : (IsF32<R>::value ? 4 : 3)) volume_small_kernel(const VolArgs<R> a, const FaceArgs<R> fa,
-                                                                     const int surf, const int epb) {
+// The work of elements [e0, e0 + epb).  FACES: the kernel evaluates the face
+// fluxes itself; otherwise the face kernel has stored them.  EARLY: the kernel
+// may have been launched early (grid_wait).
+template <typename R, int DIM, int N, int VOL, bool FACES, bool EARLY>
+__device__ __forceinline__ void small_body(const VolArgs<R> &a, const FaceArgs<R> &fa, const int surf, const int epb,
+                                           const int e0) {
   using S = Shape<DIM, N>;
   using M = SmallSmem<R, DIM, N, VOL, FACES>;
   constexpr int ND = S::ND, NEQ = S::NEQ, NFP = S::NFP, PAIRS = S::PAIRS, PRIM = M::PRIM, T = kSmallThreads;
   constexpr bool FASTABLE = !IsF32<R>::value && (VOL == VOL_CHANDRASHEKAR || VOL == VOL_RANOCHA);
-  grid_release();
+  if (EARLY) grid_release();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (dynamic_smem_bytes() < M::bytes(epb)) {
     if (threadIdx.x == 0) atomicOr(a.status, STATUS_LAUNCH);
@@ -75,7 +80,6 @@ __global__ void __launch_bounds__(kSmallThreads, FACES ? 2 : (IsF32<R>::value ? 
   R *sF = sB + epb * DIM * PAIRS * M::FP;                  // [epb][2*DIM][NEQ][NFP] face fluxes
   int *sE = reinterpret_cast<int *>(sF + (FACES ? epb * 2 * DIM * NEQ * NFP : 0));  // [epb][2*DIM] elem_face
   const int tid = threadIdx.x;
-  const int e0 = blockIdx.x * epb;
   const int cnt = min(epb, a.ne - e0);
   const long long L = (long long)a.ne * ND;
   for (int i = tid; i < N * N; i += T) sD[i] = a.ops[i];
@@ -86,7 +90,7 @@ __global__ void __launch_bounds__(kSmallThreads, FACES ? 2 : (IsF32<R>::value ? 
     const int line = p / S::NP;
     sPT[i] = (unsigned)line_node<DIM, N>(dir, line, lo) | ((unsigned)line_node<DIM, N>(dir, line, hi) << 16);
   }
-  grid_wait();  // what precedes reads the mesh only
+  if (EARLY) grid_wait();  // what precedes reads the mesh only
   if (!FACES)
     for (int i = tid; i < cnt * 2 * DIM; i += T) sE[i] = a.elem_face[(long long)e0 * 2 * DIM + i];
   // face fluxes; a boundary face's is the boundary kernel's
@@ -193,6 +197,17 @@ __global__ void __launch_bounds__(kSmallThreads, FACES ? 2 : (IsF32<R>::value ? 
     finish_node<R, DIM, N>(a, e, n, sc, a.alpha ? a.alpha[e] : 0.0, dt, f, fp, w, fl, du, bad);
   }
   if (IsF32<R>::value && bad) atomicOr(a.status, STATUS_NONPOSITIVE);
+}
+
+template <typename R, bool FACES>
+constexpr int small_min_blocks() {
+  return FACES ? 2 : (IsF32<R>::value ? 4 : 3);
+}
+
+template <typename R, int DIM, int N, int VOL, bool FACES>
+__global__ void __launch_bounds__(kSmallThreads, (small_min_blocks<R, FACES>()))
+volume_small_kernel(const VolArgs<R> a, const FaceArgs<R> fa, const int surf, const int epb) {
+  small_body<R, DIM, N, VOL, FACES, true>(a, fa, surf, epb, blockIdx.x * epb);
 }
 
 }  // namespace thx
