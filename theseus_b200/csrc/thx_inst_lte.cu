@@ -13,8 +13,8 @@ namespace thx {
 #ifdef THX_N
 LteKernels THX_XCAT3(lte_kernels, THX_DIM, THX_N)() {
   LteKernels k;
-  k.vol[0] = &launch_volume<double, THX_DIM, THX_N, VOL_LTEEC, false, false>;
-  k.vol[1] = &launch_volume<double, THX_DIM, THX_N, VOL_LTEEC, true, false>;
+  k.vol[0] = &launch_volume_lte<THX_DIM, THX_N, false>;
+  k.vol[1] = &launch_volume_lte<THX_DIM, THX_N, true>;
   k.grad = &launch_grad<double, THX_DIM, THX_N, true>;
   return k;
 }

@@ -10,13 +10,15 @@
 //                    found the factor constant (exactly) over nodes/elements.
 //
 // Kernel structure per right-hand side:
-//   NS only : grad_kernel   element-local BR1 gradient of entropy variables with
-//             the interior-face lift, converted to primitive gradients and on to
-//             the physical viscous flux, which is what the other kernels read.
+//   NS only : a gradient kernel: element-local BR1 gradient of entropy
+//             variables with the interior-face lift, converted to primitive
+//             gradients and on to the physical viscous flux (read by the face
+//             kernel) and its divergence (read by the volume kernel).
 //   always  : face_kernel   one thread per face point: F*(u-,u+,n) (- n.avg(F_v)).
-//   always  : volume_kernel one CTA per EPB elements: flux differencing with every
-//             symmetric pair evaluated once, optional subcell-FV blend, viscous
-//             divergence, surface lift from fs; writes dudt once.
+//   always  : a volume kernel (thx_volume.cuh, thx_small.cuh; LTE gas: below):
+//             flux differencing with every symmetric pair evaluated once,
+//             optional subcell-FV blend, viscous divergence, surface lift from
+//             fs; writes dudt once.  Small meshes evaluate their faces here too.
 #pragma once
 #include "thx_device.cuh"
 #include "thx_bc.cuh"
@@ -118,22 +120,19 @@ __device__ __forceinline__ void grid_start() {
   grid_wait();
 }
 
-// Shared-memory layout of the volume kernel, in elements of R:
-// [ops | prim + pair fluxes, or the viscous flux | state (NEEDQ) | metric].
-template <typename R, int DIM, int N, int VOL, bool NS, bool BLEND, int EPBX = 0>
-struct VolSmem {
-  using S = Shape<DIM, N, EPBX>;
-  static constexpr bool NEEDQ = VOL == VOL_CENTRAL;
-  static constexpr int PRIM = VOL == VOL_LTEEC ? S::NEQ + LTE_P_COUNT : nprim<R, DIM>();
+// Shared-memory layout of the LTEEC volume kernel, in doubles:
+// [ops | node data + pair fluxes, or the viscous flux | pair table | metric].
+template <int DIM, int N, bool NS>
+struct LteVolSmem {
+  using S = Shape<DIM, N>;
+  static constexpr int PRIM = S::NEQ + LTE_P_COUNT;
   static constexpr int REGION = S::EPB * (PRIM * S::ND + S::PAIRS * S::NEQ);
   static constexpr int VISC = NS ? S::EPB * DIM * (S::NEQ - 1) * S::ND : 0;
   static constexpr int SHARED = REGION > VISC ? REGION : VISC;
-  static constexpr int STATE = NEEDQ ? S::EPB * S::NEQ * S::ND : 0;
   // pair table: (lower node | upper node << 16) of every pair, per direction
-  static constexpr int PTAB = (DIM * S::PAIRS * 4 + (int)sizeof(R) - 1) / (int)sizeof(R);
+  static constexpr int PTAB = (DIM * S::PAIRS * 4 + 7) / 8;
   __host__ __device__ static constexpr size_t bytes(bool metric_per_node) {
-    return sizeof(R) * ((size_t)S::OPS + SHARED + STATE + PTAB +
-                        (size_t)S::EPB * (metric_per_node ? S::ND * DIM * DIM : DIM * DIM));
+    return 8 * ((size_t)S::OPS + SHARED + PTAB + (size_t)S::EPB * (metric_per_node ? S::ND * DIM * DIM : DIM * DIM));
   }
 };
 
@@ -193,9 +192,6 @@ __device__ __forceinline__ void surface_flux_rt(int kind, const GasT<R> &g, cons
   }
 }
 
-// One CTA's work of the volume kernel: elements [block*EPB, block*EPB + EPB).
-// Shared by the one-case kernel (block = blockIdx.x) and the batched
-// persistent kernel (block from its work list).
 // Stride (in R) between the NEQ arrays of a block's state staged in shared
 // memory: EPB*ND rounded up to 16 bytes, so every array starts 16-byte aligned.
 template <typename R, int DIM, int N, int EPBX = 0>
@@ -204,31 +200,34 @@ __host__ __device__ constexpr int stage_kstride() {
   return (int)(((size_t)S::EPB * S::ND * sizeof(R) + 15) / 16 * 16 / sizeof(R));
 }
 
-// su: the block's state staged in shared memory (array k at k*stage_kstride,
-// element el's node n at el*ND + n), or nullptr to read it from a.u.
-template <typename R, int DIM, int N, int VOL, bool NS, bool BLEND, int EPBX = 0>
-__device__ __forceinline__ void volume_body(const VolArgs<R> &a, const int block,
-                                            const R *su = nullptr) {
-  using S = Shape<DIM, N, EPBX>;
-  static_assert(VOL != VOL_LTEEC || (!BLEND && !IsF32<R>::value), "LTEEC: FP64, no blending");
-  using L_ = VolSmem<R, DIM, N, VOL, NS, BLEND, EPBX>;
+template <typename R, int DIM, int NFP>
+__device__ __forceinline__ bool lift_weight(const VolArgs<R> &a, const int fs, const int fp, R &w);
+template <typename R, int DIM, int N>
+__device__ __forceinline__ void lift_and_store(const VolArgs<R> &a, const int e, const int n, const double dt,
+                                               const int *f, const int *fp, const R *w, const R (*fl)[DIM + 2], R *du,
+                                               bool &bad);
+
+// One CTA's work of the LTEEC volume kernel: elements [block*EPB, block*EPB +
+// EPB), one thread per symmetric pair, its flux passed through shared memory to
+// one thread per node (a thread's pair holds the whole register budget).
+template <int DIM, int N, bool NS>
+__device__ __forceinline__ void lte_volume_body(const VolArgs<double> &a, const int block) {
+  using R = double;
+  using S = Shape<DIM, N>;
+  using L_ = LteVolSmem<DIM, N, NS>;
   constexpr int ND = S::ND, NEQ = S::NEQ, EPB = S::EPB, NPRIM = L_::PRIM, PAIRS = S::PAIRS;
   constexpr int MB = DIM * DIM;
-  constexpr bool NEEDQ = L_::NEEDQ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (a.skip_block && a.skip_block[block]) return;  // block-uniform: before any barrier
   if (dynamic_smem_bytes() < L_::bytes(a.met_ns != 0)) {
     if (threadIdx.x == 0) atomicOr(a.status, STATUS_LAUNCH);
     return;
   }
-  // [ops | prim | pair fluxes | state (NEEDQ) | metric]; the viscous flux of the
-  // NS phase reuses the prim + pair-flux region, the FV rate the pair fluxes.
+  // the viscous flux of the NS phase reuses the node data + pair-flux region
   R *sOps = reinterpret_cast<R *>(smem_raw);              // 2*N*N + N (padded)
   R *sPrim = sOps + S::OPS;                               // [EPB][NPRIM][ND]
   R *sFB = sPrim + EPB * NPRIM * ND;                      // [EPB][PAIRS][NEQ]
-  R *sQ = sPrim + L_::SHARED;                             // [EPB][NEQ][ND] if NEEDQ
-  unsigned *sPT = reinterpret_cast<unsigned *>(sQ + L_::STATE);  // [DIM][PAIRS]
-  R *sMet = sQ + L_::STATE + L_::PTAB;                    // per node or once per element
+  unsigned *sPT = reinterpret_cast<unsigned *>(sPrim + L_::SHARED);  // [DIM][PAIRS]
+  R *sMet = sPrim + L_::SHARED + L_::PTAB;                // per node or once per element
   R *sFv = sPrim;                                         // [EPB][DIM][NEQ-1][ND] (NS)
   const int mns = a.met_ns != 0 ? MB : 0;                 // metric node stride in smem
   const int mbk = a.met_ns != 0 ? ND * MB : MB;           // metric element block in smem
@@ -246,7 +245,6 @@ __device__ __forceinline__ void volume_body(const VolArgs<R> &a, const int block
   }
   const R *sD2 = sOps;
   const R *sDh = sOps + N * N;
-  const R *sW = sOps + 2 * N * N;
 
   // stage states, node data and metric
   const int el = tid / ND, n = tid % ND;
@@ -254,49 +252,29 @@ __device__ __forceinline__ void volume_body(const VolArgs<R> &a, const int block
   const bool active = (el < EPB) && (e < a.ne);
   if (active) {
     R q[NEQ];
-    if (su) {
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) q[k] = su[k * stage_kstride<R, DIM, N, EPBX>() + el * ND + n];
-    } else {
+    for (int k = 0; k < NEQ; ++k) q[k] = a.u[k * L + (long long)e * ND + n];
+    // conserved state, recovered T, its table cell and the pressure
+    const double T = a.gas.Tn[(long long)e * ND + n];
+    const LteEval sv = lte_at_cell(a.gas.lte, q[0], T, a.gas.Cn[(long long)e * ND + n]);
+    R pr[NPRIM];
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) q[k] = a.u[k * L + (long long)e * ND + n];
-    }
-    if constexpr (VOL == VOL_LTEEC) {
-      // conserved state, recovered T, its table cell and the pressure
-      const double T = a.gas.Tn[(long long)e * ND + n];
-      const LteEval sv = lte_at_cell(a.gas.lte, q[0], T, a.gas.Cn[(long long)e * ND + n]);
-      R pr[NPRIM];
+    for (int k = 0; k < NEQ; ++k) pr[k] = q[k];
+    pr[NEQ + LTE_P_T] = T;
+    pr[NEQ + LTE_P_XI] = sv.xi;
+    pr[NEQ + LTE_P_ETA] = sv.eta;
+    pr[NEQ + LTE_P_DR] = sv.cell.dr;
+    pr[NEQ + LTE_P_DT] = sv.cell.dt;
+    pr[NEQ + LTE_P_OFF] = (double)sv.cell.off;
+    const LteJet jv = lte_jet(a.gas.lte, sv);
+    pr[NEQ + LTE_P_H] = jv.H;
+    pr[NEQ + LTE_P_HR] = jv.Hr;
+    pr[NEQ + LTE_P_HT] = jv.HT;
+    pr[NEQ + LTE_P_HRR] = jv.Hrr;
+    pr[NEQ + LTE_P_HRT] = jv.HrT;
 #pragma unroll
-      for (int k = 0; k < NEQ; ++k) pr[k] = q[k];
-      pr[NEQ + LTE_P_T] = T;
-      pr[NEQ + LTE_P_XI] = sv.xi;
-      pr[NEQ + LTE_P_ETA] = sv.eta;
-      pr[NEQ + LTE_P_DR] = sv.cell.dr;
-      pr[NEQ + LTE_P_DT] = sv.cell.dt;
-      pr[NEQ + LTE_P_OFF] = (double)sv.cell.off;
-      const LteJet jv = lte_jet(a.gas.lte, sv);
-      pr[NEQ + LTE_P_H] = jv.H;
-      pr[NEQ + LTE_P_HR] = jv.Hr;
-      pr[NEQ + LTE_P_HT] = jv.HT;
-      pr[NEQ + LTE_P_HRR] = jv.Hrr;
-      pr[NEQ + LTE_P_HRT] = jv.HrT;
-#pragma unroll
-      for (int k = 0; k < NPRIM; ++k) sPrim[(el * NPRIM + k) * ND + n] = pr[k];
-      if (!sv.valid || !(q[0] > 0.0)) atomicOr(a.status, STATUS_EOS);
-    } else {
-      R pr[NPRIM];
-      node_prims<R, DIM, VOL>(a.gas, q, pr);
-#pragma unroll
-      for (int k = 0; k < NPRIM; ++k) sPrim[(el * NPRIM + k) * ND + n] = pr[k];
-      if (NEEDQ) {
-#pragma unroll
-        for (int k = 0; k < NEQ; ++k) sQ[(el * NEQ + k) * ND + n] = q[k];
-      }
-      // FP64 path: positivity of the state read here.  FP32-mixed: checked
-      // on the FP64 master state instead (to_working, the RK stage epilogue)
-      if (!IsF32<R>::value && (!(pr[0] > R(0)) || !(pr[DIM + 1] > R(0))))
-        atomicOr(a.status, STATUS_NONPOSITIVE);
-    }
+    for (int k = 0; k < NPRIM; ++k) sPrim[(el * NPRIM + k) * ND + n] = pr[k];
+    if (!sv.valid || !(q[0] > 0.0)) atomicOr(a.status, STATUS_EOS);
     if (mns != 0 || n == 0) {
       const R *mp = a.met + (long long)e * a.met_es + (long long)n * a.met_ns;
 #pragma unroll
@@ -311,10 +289,8 @@ __device__ __forceinline__ void volume_body(const VolArgs<R> &a, const int block
 #pragma unroll
   for (int k = 0; k < NEQ; ++k) rate[k] = R(0);
 
-  // directions unrolled: 2 % faster than rolled (32^3 p=4, FP64 and FP32);
-  // rolled for the LTEEC flux, whose spills it would multiply
-  constexpr int DIR_UNROLL = VOL == VOL_LTEEC ? 1 : DIM;
-#pragma unroll DIR_UNROLL
+  // rolled: unrolling would multiply the flux's spills
+#pragma unroll 1
   for (int dir = 0; dir < DIM; ++dir) {
     // pair phase: every symmetric pair once, in (lower, upper) order
     for (int t = tid; t < EPB * PAIRS; t += S::THREADS) {  // launched with S::THREADS
@@ -337,27 +313,12 @@ __device__ __forceinline__ void volume_body(const VolArgs<R> &a, const int block
         for (int d = 0; d < DIM; ++d)
           met[d] = R(0.5) * (sMet[pel * mbk + na * mns + dir * DIM + d] + sMet[pel * mbk + nb * mns + dir * DIM + d]);
       }
-      if constexpr (VOL == VOL_LTEEC) {
-        // include/LTEECFlux.hpp:11-84: the averaged metric passed as both rows
-        // (0.5*(m+m) == m exactly)
-        const LteEval sa = lte_unpack(A + NEQ, A[0], a.gas.lte.nx);
-        const LteEval sb = lte_unpack(B + NEQ, B[0], a.gas.lte.nx);
-        lte_ec_flux<DIM, false>(a.gas.lte, A, B, sa, sb, lte_unpack_jet(A + NEQ),
-                                lte_unpack_jet(B + NEQ), met, met, F);
-      } else if (VOL == VOL_CHANDRASHEKAR) vol_chandrashekar<R, DIM>(a.gas, A, B, met, F);
-      else if (VOL == VOL_RANOCHA) vol_ranocha<R, DIM>(a.gas, A, B, met, F);
-      else if (VOL == VOL_PIROZZOLI) vol_pirozzoli<R, DIM>(a.gas, A, B, met, F);
-      else {
-        R RA[NEQ], RB[NEQ], QA[NEQ], QB[NEQ];
-#pragma unroll
-        for (int k = 0; k < NEQ; ++k) {
-          RA[k] = sQ[(pel * NEQ + k) * ND + na];
-          RB[k] = sQ[(pel * NEQ + k) * ND + nb];
-        }
-        reconstruct<R, DIM>(a.gas, RA, QA);
-        reconstruct<R, DIM>(a.gas, RB, QB);
-        vol_central<R, DIM>(QA, QB, A, B, met, F);
-      }
+      // include/LTEECFlux.hpp:11-84: the averaged metric passed as both rows
+      // (0.5*(m+m) == m exactly)
+      const LteEval sa = lte_unpack(A + NEQ, A[0], a.gas.lte.nx);
+      const LteEval sb = lte_unpack(B + NEQ, B[0], a.gas.lte.nx);
+      lte_ec_flux<DIM, false>(a.gas.lte, A, B, sa, sb, lte_unpack_jet(A + NEQ),
+                              lte_unpack_jet(B + NEQ), met, met, F);
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) sFB[(pel * PAIRS + pidx) * NEQ + k] = F[k];
     }
@@ -380,23 +341,13 @@ __device__ __forceinline__ void volume_body(const VolArgs<R> &a, const int block
   }
 
   R du[NEQ];
+  bool unused = false;
   R J = R(1);
   if (active) {
     J = a.jac[(long long)e * a.jac_es + (long long)n * a.jac_ns];
     const R s = R(-1) / J;
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) du[k] = s * rate[k];
-  }
-
-  // subcell finite-volume blend (include/EulerOperator_impl.hpp:134-152):
-  // fv_kernel has stored the FV rate of every blended element
-  if (BLEND && a.alpha != nullptr && active) {
-    const double al = a.alpha[e];
-    if (al > 1e-16) {
-      const R af = (R)al, ad = (R)(1.0 - al);
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) du[k] = ad * du[k] + af * a.fvrate[((long long)e * NEQ + k) * ND + n];
-    }
   }
 
   if (NS) {
@@ -447,96 +398,21 @@ __device__ __forceinline__ void volume_body(const VolArgs<R> &a, const int block
   }
 
   if (!active) return;
-  // surface lift: interior faces summed first, then added (restr_f
-  // transpose; +=); then the boundary faces the same way (restr_b)
-#pragma unroll 1
-  for (int pass = 0; pass < ((!IsF32<R>::value && a.bw) ? 2 : 1); ++pass) {
-    R acc[NEQ];
+  // surface lift (every face is interior) and Runge-Kutta stage
+  int f[DIM], fp[DIM];
+  R w[DIM], fl[DIM][NEQ];
 #pragma unroll
-    for (int k = 0; k < NEQ; ++k) acc[k] = R(0);
-    bool any = false;
+  for (int d = 0; d < DIM; ++d) {
+    f[d] = c[d] == 0 || c[d] == N - 1 ? a.elem_face[e * 2 * DIM + 2 * d + (c[d] == N - 1 ? 1 : 0)] : -1;
+    fp[d] = face_point<DIM, N>(d, c);
+    const bool in = lift_weight<R, DIM, S::NFP>(a, f[d], fp[d], w[d]);
 #pragma unroll
-    for (int dir = 0; dir < DIM; ++dir) {
-      const int me = c[dir];
-      if (me != 0 && me != N - 1) continue;
-      const int lf = 2 * dir + (me == N - 1 ? 1 : 0);
-      const int fs = a.elem_face[e * 2 * DIM + lf];
-      if (fs < 0) continue;
-      const int f = fs >> 1, side = fs & 1;
-      const int fp = face_point<DIM, N>(dir, c);
-      R w;
-      if (!IsF32<R>::value && a.bw && f >= a.nf_int) {  // boundary face (FP64 only)
-        if (pass == 0) continue;
-        w = -a.bw[(long long)(f - a.nf_int) * S::NFP + fp];
-      } else {
-        if (pass == 1) continue;
-        const long long wi = (long long)f * a.w_fs + (long long)fp * a.w_ps;
-        w = side == 0 ? -a.wm[wi] : a.wp[wi];
-      }
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) acc[k] += w * a.fstar[((long long)f * NEQ + k) * S::NFP + fp];
-      any = true;
-    }
-    if (any) {
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) du[k] += acc[k];
+    for (int k = 0; k < NEQ; ++k) {
+      fl[d][k] = R(0);
+      if (in) fl[d][k] = a.fstar[((long long)(f[d] >> 1) * NEQ + k) * S::NFP + fp[d]];
     }
   }
-  const long long base = (long long)e * ND + n;
-  if (a.stage == 0) {
-    if (a.du64) {
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) a.du64[k * L + base] = (double)du[k];
-    } else {
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) a.du[k * L + base] = du[k];
-    }
-  } else {
-    // fused SSP-RK3 stage in the arithmetic order of mfem::RK3SSPSolver::Step
-    const double dt = a.dt_dev ? *a.dt_dev : a.dt;
-    // every load before the first store: the state arrays may alias as far
-    // as the compiler knows, so interleaving would serialise the round trips
-    double umv[NEQ], yv[NEQ];
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k) {
-      const long long i = k * L + base;
-      umv[k] = a.um[i];
-      yv[k] = a.stage == 1 ? 0.0 : a.y[i];
-    }
-    double ynew[NEQ];
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k) {
-      const double kk = (double)du[k];
-      double y;
-      if (a.stage == 1) {
-        y = umv[k] + dt * kk;
-      } else if (a.stage == 2) {
-        y = yv[k] + dt * kk;
-        y = 0.75 * umv[k] + 0.25 * y;
-      } else {
-        y = yv[k] + dt * kk;
-        y = (1.0 / 3.0) * umv[k] + (2.0 / 3.0) * y;
-        // a device-side step of 0 (a finished time loop, or no valid rate)
-        // leaves the state exactly as it was
-        if (a.dt_dev && dt == 0.0) y = umv[k];
-      }
-      ynew[k] = y;
-    }
-#pragma unroll
-    for (int k = 0; k < NEQ; ++k) {
-      const long long i = k * L + base;
-      if (a.stage == 3) {
-        if (!(a.dt_dev && dt == 0.0)) a.um[i] = ynew[k];
-      } else {
-        a.yo[i] = ynew[k];
-      }
-      if (a.yf) a.yf[i] = (float)(ynew[k] - a.off[k]);
-    }
-    if constexpr (IsF32<R>::value) {
-      // FP32-mixed: positivity of the new FP64 stage state, in FP64
-      if (!fp64_state_positive<DIM>(ynew, (double)a.gas.gm1)) atomicOr(a.status, STATUS_NONPOSITIVE);
-    }
-  }
+  lift_and_store<R, DIM, N>(a, e, n, a.stage == 0 ? 0.0 : a.dt_dev ? *a.dt_dev : a.dt, f, fp, w, fl, du, unused);
 }
 
 template <int DIM, int SURF>
@@ -650,18 +526,13 @@ __global__ void __launch_bounds__(Shape<DIM, N>::THREADS) fv_kernel(const VolArg
   fv_body<R, DIM, N>(a, blockIdx.x);
 }
 
-template <typename R, int DIM, int N, int VOL, bool NS, bool BLEND>
-__global__ void __launch_bounds__(Shape<DIM, N>::THREADS) volume_kernel(const VolArgs<R> a) {
-  volume_body<R, DIM, N, VOL, NS, BLEND>(a, blockIdx.x);
-}
-
-// The same with MINB CTAs per SM required.  FP64 takes four (8 % faster
-// than the compiler's three); the LTEEC flux takes two (left alone the
-// compiler gives it the whole register file and one CTA).
-template <typename R, int DIM, int N, int VOL, bool NS, bool BLEND, int MINB>
-__global__ void __launch_bounds__(Shape<DIM, N>::THREADS, MINB) volume_kernel_mb(const VolArgs<R> a) {
+// The LTEEC volume kernel, two CTAs per SM required (left alone the compiler
+// gives it the whole register file and one CTA; one element per CTA with three
+// or four CTAs per SM is 2 and 4 % slower at 24^3 p=4).
+template <int DIM, int N, bool NS>
+__global__ void __launch_bounds__(Shape<DIM, N>::THREADS, 2) volume_kernel_lte(const VolArgs<double> a) {
   grid_start();
-  volume_body<R, DIM, N, VOL, NS, BLEND>(a, blockIdx.x);
+  lte_volume_body<DIM, N, NS>(a, blockIdx.x);
 }
 
 }  // namespace thx
@@ -826,11 +697,6 @@ volume_tma_kernel(const VolArgs<R> a) {
       if (pending[q]) mbar_wait_bounded(&bars[q], phase[q]);
   }
 }
-
-template <typename R, int VOL, bool BLEND>
-struct VolMinBlocks {
-  static constexpr int value = VOL == VOL_LTEEC ? 2 : (!IsF32<R>::value ? 4 : 6);
-};
 
 // ---------------------------------------------------------------------------
 template <typename R>

@@ -51,31 +51,17 @@ template <typename R>
 using FaceBatchLaunch = cudaError_t (*)(const FaceArgs<R> *, const BatchWork *, const int *, int,
                                         cudaStream_t, int);
 
-template <typename R, int DIM, int N, int VOL, bool NS, bool BLEND>
-constexpr size_t volume_smem_bytes(bool metric_per_node) {
-  return VolSmem<R, DIM, N, VOL, NS, BLEND>::bytes(metric_per_node);
-}
-
-template <typename R, int DIM, int N, int VOL, bool NS, bool BLEND>
-cudaError_t launch_volume(const VolArgs<R> &a, cudaStream_t s, int prepare) {
+// The LTEEC volume kernel.
+template <int DIM, int N, bool NS>
+cudaError_t launch_volume_lte(const VolArgs<double> &a, cudaStream_t s, int prepare) {
   using S = Shape<DIM, N>;
-  static_assert(S::PAIRS >= S::ND, "subcell FV rate aliases the pair-flux buffer");
-  constexpr int MINB = VolMinBlocks<R, VOL, BLEND>::value;
-  if (prepare) {
-    const int bytes = (int)volume_smem_bytes<R, DIM, N, VOL, NS, BLEND>(true);
-    if constexpr (MINB > 0)
-      return cudaFuncSetAttribute(volume_kernel_mb<R, DIM, N, VOL, NS, BLEND, MINB>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    else
-      return cudaFuncSetAttribute(volume_kernel<R, DIM, N, VOL, NS, BLEND>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  }
+  using M = LteVolSmem<DIM, N, NS>;
+  if (prepare)
+    return cudaFuncSetAttribute(volume_kernel_lte<DIM, N, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)M::bytes(true));
   if (a.ne <= 0) return cudaSuccess;
-  const size_t smem = volume_smem_bytes<R, DIM, N, VOL, NS, BLEND>(a.met_ns != 0);
-  const int grid = (a.ne + S::EPB - 1) / S::EPB;
-  if constexpr (MINB > 0) return launch_early(volume_kernel_mb<R, DIM, N, VOL, NS, BLEND, MINB>, grid, S::THREADS, smem, s, a);
-  else volume_kernel<R, DIM, N, VOL, NS, BLEND><<<grid, S::THREADS, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_early(volume_kernel_lte<DIM, N, NS>, (a.ne + S::EPB - 1) / S::EPB, S::THREADS, M::bytes(a.met_ns != 0),
+                      s, a);
 }
 
 // The line kernel (ideal gas): one thread per tensor line.

@@ -308,7 +308,7 @@ template <typename R, int DIM, int N>
 __device__ __forceinline__ void finish_node(const VolArgs<R> &a, const int e, const int n, const R sc,
                                             const double al, const double dt, const int *f, const int *fp,
                                             const R *w, const R (*fl)[DIM + 2], R *du, bool &bad) {
-  constexpr int ND = DIM == 2 ? N * N : N * N * N, NFP = ND / N, NEQ = DIM + 2;
+  constexpr int ND = DIM == 2 ? N * N : N * N * N, NEQ = DIM + 2;
   const long long L = (long long)a.ne * ND, gi = (long long)e * ND + n;
   R dv[NEQ - 1];
 #pragma unroll
@@ -331,6 +331,17 @@ __device__ __forceinline__ void finish_node(const VolArgs<R> &a, const int e, co
 #pragma unroll
     for (int k = 0; k < NEQ - 1; ++k) du[1 + k] += sc * dv[k];
   }
+  lift_and_store<R, DIM, N>(a, e, n, dt, f, fp, w, fl, du, bad);
+}
+
+// The last of finish_node: the surface lift of du, and the rate or the
+// Runge-Kutta stage.
+template <typename R, int DIM, int N>
+__device__ __forceinline__ void lift_and_store(const VolArgs<R> &a, const int e, const int n, const double dt,
+                                               const int *f, const int *fp, const R *w, const R (*fl)[DIM + 2], R *du,
+                                               bool &bad) {
+  constexpr int ND = DIM == 2 ? N * N : N * N * N, NFP = ND / N, NEQ = DIM + 2;
+  const long long L = (long long)a.ne * ND, gi = (long long)e * ND + n;
   // interior faces summed first, then added (restr_f transpose; +=); then the
   // boundary faces the same way (restr_b)
 #pragma unroll
