@@ -421,7 +421,7 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
                : (cfg->volume_flux == THX_FLUX_PIROZZOLI)   ? VOL_PIROZZOLI
                                                             : VOL_CENTRAL;
   h->lte = table != nullptr;
-  h->small = h->lte || (h->mixed && (h->blend || h->nbf > 0)) || cfg->volume_staging == 1 ? 0 : small_mesh(g->dim, h->N, h->ne);
+  h->small = h->lte || (h->mixed && (h->blend || h->nbf > 0)) || cfg->volume_staging == 1 ? 0 : small_mesh(g->dim, h->N, h->ne, h->mixed);
   // a batched case's last steps: its buffers are those of the batched kernels
   if (h->pool && h->small > 1) h->small = 1;
   if (h->lte) {

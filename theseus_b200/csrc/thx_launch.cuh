@@ -84,12 +84,12 @@ using SmallLaunch = cudaError_t (*)(const VolArgs<R> &, const FaceArgs<R> &, int
 template <typename R, int DIM, int N, int VOL, bool FACES>
 cudaError_t launch_volume_small(const VolArgs<R> &a, const FaceArgs<R> &fa, int surf, cudaStream_t s, int prepare) {
   using M = SmallSmem<R, DIM, N, VOL, FACES>;
-  const int epb = small_epb(DIM, N, a.ne, FACES);
-  static_assert(M::bytes(small_epb(DIM, N, 1 << 30, FACES)) <= 200 * 1024, "shared memory");
+  const int epb = small_epb(DIM, N, a.ne, FACES, IsF32<R>::value);
+  static_assert(M::bytes(small_epb(DIM, N, 1 << 30, FACES, IsF32<R>::value)) <= 200 * 1024, "shared memory");
   if (prepare)
     return cudaFuncSetAttribute(volume_small_kernel<R, DIM, N, VOL, FACES>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)M::bytes(small_epb(DIM, N, 1 << 30, FACES)));
+                                (int)M::bytes(small_epb(DIM, N, 1 << 30, FACES, IsF32<R>::value)));
   if (a.ne <= 0) return cudaSuccess;
   return launch_early(volume_small_kernel<R, DIM, N, VOL, FACES>, (a.ne + epb - 1) / epb, kSmallThreads, M::bytes(epb), s, a, fa, surf, epb);
 }

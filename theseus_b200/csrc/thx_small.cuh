@@ -16,13 +16,13 @@ constexpr int kSmallThreads = 256;
 constexpr int kSmallSMs = 148;
 
 // Elements per CTA.  With the face terms: spread over the SMs, up to about two
-// pairs per thread.  Without: over three CTAs per SM (all resident), up to a
-// node per thread.
-__host__ constexpr int small_epb(int dim, int N, int ne, bool faces) {
+// pairs per thread.  Without: over the CTAs that are resident at once, three
+// per SM in FP64 and four in FP32, up to a node per thread.
+__host__ constexpr int small_epb(int dim, int N, int ne, bool faces, bool f32) {
   const int nd = dim == 2 ? N * N : N * N * N;
   const int pairs = dim * (nd / N) * (N * (N - 1) / 2);
   const int most = faces ? 2 * kSmallThreads / pairs : kSmallThreads / nd;
-  const int ctas = faces ? kSmallSMs : 3 * kSmallSMs;
+  const int ctas = faces ? kSmallSMs : (f32 ? 4 : 3) * kSmallSMs;
   const int spread = (ne + ctas - 1) / ctas;
   const int epb = spread < most ? spread : most;
   return epb > 1 ? epb : 1;
@@ -30,15 +30,15 @@ __host__ constexpr int small_epb(int dim, int N, int ne, bool faces) {
 
 // Which volume kernel a mesh takes: 2 this one with the face terms, 1 this one
 // after the face kernel, 0 the line kernel after the face kernel.  The first
-// two while their CTAs are resident at once (two and three per SM, by their
-// registers); beyond, the line kernel's fewer instructions outweigh its longer
+// two while their CTAs are resident at once (two, and three or four per SM, by
+// their registers); beyond, the line kernel's fewer instructions outweigh its longer
 // chains.  RK3 stage of the 2-D Euler vortex, FP64, first / second / line
 // kernel: 32^2 p=3 9.8 / 13.7 / 21.6 us, 48^2 10.3 / 14.4 / 22.0, 64^2 16.4 /
 // 15.8 / 22.2, 96^2 28.7 / 24.1 / 22.6, 128^2 44.3 / 32.8 / 28.5; 3-D p=3 5^3
 // 10.3 / 16.4 / 28.7, 7^3 18.5 / 16.4 / 28.7, 16^3 110 / 85 / 51.
-__host__ constexpr int small_mesh(int dim, int N, int ne) {
-  const int e2 = small_epb(dim, N, ne, true), e1 = small_epb(dim, N, ne, false);
-  return (ne + e2 - 1) / e2 <= 2 * kSmallSMs ? 2 : (ne + e1 - 1) / e1 <= 3 * kSmallSMs ? 1 : 0;
+__host__ constexpr int small_mesh(int dim, int N, int ne, bool f32) {
+  const int e2 = small_epb(dim, N, ne, true, f32), e1 = small_epb(dim, N, ne, false, f32);
+  return (ne + e2 - 1) / e2 <= 2 * kSmallSMs ? 2 : (ne + e1 - 1) / e1 <= (f32 ? 4 : 3) * kSmallSMs ? 1 : 0;
 }
 
 template <typename R, int DIM, int N, int VOL, bool FACES>
