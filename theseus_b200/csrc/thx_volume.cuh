@@ -64,60 +64,26 @@ struct LineSmem {
 // their product serves both logarithmic means, and each quotient is rounded
 // from it by the residual correction q + (a - b q) y (P. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990), which returns the correctly rounded a / b unless the
-// quotient lies within about 2^-27 ulp of a rounding boundary.  The results
-// are those of the separate divisions.
+// processor", 1990).  From y = (1 + d)/b the corrected quotient is off by at
+// most |d| (2^53 |d| + 1) ulp before its rounding, below 2^-34 ulp for the
+// least accurate reciprocal used (4e-14): it is the correctly rounded a / b
+// but for quotients that close to a rounding boundary.  Everything else -- the
+// branch variable, the series, the logarithm -- is formed as log_mean and the
+// fluxes of thx_device.cuh form it, so the results do not depend on which of
+// the two a CTA takes.  (The branch variable from a reciprocal instead of a
+// quotient, and the series with fused multiply-adds, would be up to 3 % faster
+// and change the last bit of about one mean in 10^4.)
 
-// 1/x to about an ulp for normal x: the hardware's 20-bit start and one
-// third-order Newton step.
-__device__ __forceinline__ double rcp_refined(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = __fma_rn(-x, y, 1.0);
-  return __fma_rn(y, __fma_rn(e, e, e), y);
-}
-// a / b from y ~ 1/b
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  const double q = a * y;
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-
-// log(x) for normal positive x: x = 2^k m, m in [sqrt(1/2), sqrt(2)), and
-// log m = 2 artanh(g), g = (m - 1)/(m + 1), by its series (g^2 < 0.0295; the
-// terms left out are below 2e-17).
-__device__ __forceinline__ double log_normal(double x) {
-  const int hi = __double2hiint(x);
-  const int k = (hi - 0x3FE6A09E) >> 20;
-  const double m = __hiloint2double(hi - (k << 20), __double2loint(x));
-  const double b = m + 1.0;
-  const double g = div_by(m - 1.0, b, rcp_refined(b));
-  const double u = g * g;
-  double s = 1.0 / 23;
-  s = __fma_rn(s, u, 1.0 / 21);
-  s = __fma_rn(s, u, 1.0 / 19);
-  s = __fma_rn(s, u, 1.0 / 17);
-  s = __fma_rn(s, u, 1.0 / 15);
-  s = __fma_rn(s, u, 1.0 / 13);
-  s = __fma_rn(s, u, 1.0 / 11);
-  s = __fma_rn(s, u, 1.0 / 9);
-  s = __fma_rn(s, u, 1.0 / 7);
-  s = __fma_rn(s, u, 1.0 / 5);
-  s = __fma_rn(s, u, 1.0 / 3);
-  const double t = g + g, kd = (double)k;
-  // log 2 in two parts, the first with trailing zeros: k * hi is exact
-  return __fma_rn(kd, 0x1.62e42fefa3p-1, __fma_rn(t, s * u, kd * 0x1.3de6af278ece6p-42) + t);
-}
-
-// log_mean(x, y) and its reciprocal (to an ulp or two, for div_by), given
+// log_mean(x, y) and its reciprocal (to a few ulp, for div_by), given
 // rx ~ 1/x, s = x + y and rs ~ 1/s.
 template <int MODE>
 __device__ __forceinline__ void log_mean_rcp(double x, double y, double s, double rx, double rs, double &lm,
                                              double &inv) {
   const double xi = div_by(y, x, rx);
   const double v = x * rs;  // 1/(xi + 1)
-  const double u = (xi * (xi - 2.0) + 1.0) * (v * v);
+  const double u = div_by(xi * (xi - 2.0) + 1.0, xi * (xi + 2.0) + 1.0, v * v);
   if (MODE == LM_SERIES || u < 1e-4) {
-    const double z = u * __fma_rn(u, __fma_rn(15.0, u, 21.0), 35.0);
+    const double z = u * (35.0 + u * (21.0 + 15.0 * u));
     const double denom = 105.0 + z;
     // 1/denom from its expansion about 1/105 (z < 0.0036: to 4e-14)
     constexpr double c = 1.0 / 105.0;
