@@ -339,21 +339,21 @@ class Engine final : public EngineBase {
   // kernels of the running groups to leave an SM.
   int upload_working_copy(thx_operator_s *h, const double *u0) {
     const long long L = h->L;
-    const int neq = h->neq, dim = h->dim;
+    const int neq = h->neq;
     // straight into the pinned ring, without a buffer of its own
-    int st = ring_.fill(h->yf, (size_t)L * neq * sizeof(float), setup_, [&](void *to) {
-      for (int k = 0; k < neq; ++k) {
+    int st = ring_.fill(h->yf, sizeof(float), (size_t)L * neq, setup_, [&](void *to, size_t first, size_t n) {
+      float *__restrict__ dst = (float *)to;
+      for (size_t i = first; i < first + n;) {
+        const size_t k = i / L, end = std::min((k + 1) * (size_t)L, first + n);
         const double o = h->off.v[k];
-        const double *__restrict__ src = u0 + (size_t)k * L;
-        float *__restrict__ dst = (float *)to + (size_t)k * L;
-        for (long long i = 0; i < L; ++i) dst[i] = (float)(src[i] - o);
+        for (; i < end; ++i) dst[i - first] = (float)(u0[i] - o);
       }
     });
     // no early exit: the loop stays vectorised
     int bad = 0;
     const double gm1 = h->g64.gm1;
-    const double *rho = u0, *mx = u0 + L, *my = u0 + 2 * L, *mz = dim == 3 ? u0 + 3 * L : nullptr;
-    const double *en = u0 + (size_t)(dim + 1) * L;
+    const double *rho = u0, *mx = u0 + L, *my = u0 + 2 * L, *mz = h->dim == 3 ? u0 + 3 * L : nullptr;
+    const double *en = u0 + (size_t)(h->dim + 1) * L;
     for (long long i = 0; i < L; ++i) {
       double m2 = 0.0 + mx[i] * mx[i];
       m2 += my[i] * my[i];

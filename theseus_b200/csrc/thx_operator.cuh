@@ -9,12 +9,8 @@
 #include <vector>
 
 #include <cstdio>
-#include <deque>
-#include <mutex>
 
-#include <chrono>
-
-#include "thx_ring.h"
+#include "thx_staging.h"
 
 namespace thx {
 
@@ -32,96 +28,28 @@ inline int cuda_failed(cudaError_t e, const char *call, int status = THX_ERR_CUD
     if (thx_e_ != cudaSuccess) return thx::cuda_failed(thx_e_, #call); \
   } while (0)
 
-// Pinned host staging ring for stream-ordered uploads: a copy is written into
-// the ring on the host and sent with cudaMemcpyAsync, so the call neither
-// waits for the stream nor goes through the driver's pageable path.  Space
-// is reclaimed in FIFO order once each copy's event has completed.
-class HostRing {
- public:
-  ~HostRing() {
-    for (cudaEvent_t ev : busy_) cudaEventDestroy(ev);
-    for (cudaEvent_t ev : spare_) cudaEventDestroy(ev);
-    if (buf_) cudaFreeHost(buf_);
+// Device calls of the pinned staging ring of the uploads (thx_staging.h).
+struct CudaStaging {
+  using Stream = cudaStream_t;
+  using Event = cudaEvent_t;
+  static constexpr int kNoSpace = THX_ERR_OUT_OF_MEMORY;
+  static int status(cudaError_t e, const char *call) { return e == cudaSuccess ? THX_OK : cuda_failed(e, call); }
+  static int alloc(void **p, size_t bytes) {
+    return status(cudaHostAlloc(p, bytes, cudaHostAllocDefault), "cudaHostAlloc(upload ring)");
   }
-  int init(size_t bytes) {
-    if (cudaHostAlloc((void **)&buf_, bytes, cudaHostAllocDefault) != cudaSuccess) {
-      cudaGetLastError();
-      buf_ = nullptr;
-      return THX_ERR_OUT_OF_MEMORY;
-    }
-    space_.reset(bytes);
-    return THX_OK;
+  static void free(void *p) { cudaFreeHost(p); }
+  static int copy(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+    return status(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync(upload)");
   }
-  // host -> device copy of `bytes` on stream s through the ring (copies of
-  // more than half the ring go directly)
-  int copy(void *dst, const void *src, size_t bytes, cudaStream_t s) {
-    if (!fits(bytes)) {
-      const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
-      return e == cudaSuccess ? THX_OK : cuda_failed(e, "cudaMemcpyAsync(upload)");
-    }
-    return fill(dst, bytes, s, [&](void *to) { std::memcpy(to, src, bytes); });
+  static int create(cudaEvent_t *ev) {
+    return status(cudaEventCreateWithFlags(ev, cudaEventDisableTiming), "cudaEventCreate(upload ring)");
   }
-  // the same with the bytes written by write(to), in the ring where they fit
-  template <typename F>
-  int fill(void *dst, size_t bytes, cudaStream_t s, F &&write) {
-    if (!fits(bytes)) {
-      std::vector<unsigned char> own(bytes);
-      write(own.data());
-      const cudaError_t e = cudaMemcpyAsync(dst, own.data(), bytes, cudaMemcpyHostToDevice, s);
-      return e == cudaSuccess ? THX_OK : cuda_failed(e, "cudaMemcpyAsync(upload)");
-    }
-    std::lock_guard<std::mutex> lock(mu_);
-    const size_t need = (bytes + 255) & ~size_t(255);
-    size_t off;
-    const auto t0 = std::chrono::steady_clock::now();
-    while (!space_.place(need, &off)) {  // wait for the oldest copy
-      const cudaError_t e = cudaEventSynchronize(busy_.front());
-      if (e != cudaSuccess) return cuda_failed(e, "cudaEventSynchronize(upload ring)");
-      spare_.push_back(busy_.front());
-      busy_.pop_front();
-      space_.pop();
-    }
-    const auto t1 = std::chrono::steady_clock::now();
-    write(buf_ + off);
-    const auto t2 = std::chrono::steady_clock::now();
-    wait_s_ += std::chrono::duration<double>(t1 - t0).count();
-    copy_s_ += std::chrono::duration<double>(t2 - t1).count();
-    cudaError_t e = cudaMemcpyAsync(dst, buf_ + off, bytes, cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return cuda_failed(e, "cudaMemcpyAsync(upload ring)");
-    cudaEvent_t ev;
-    if (!spare_.empty()) {
-      ev = spare_.back();
-      spare_.pop_back();
-    } else if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) {
-      return cuda_failed(e, "cudaEventCreate(upload ring)");
-    }
-    // the span is live from here on: its bytes are read by the queued copy
-    busy_.push_back(ev);
-    space_.push(off, need);
-    if ((e = cudaEventRecord(ev, s)) != cudaSuccess) {
-      // unrecorded: the event would report complete at once, so wait for the
-      // stream before the span can be reused
-      cudaStreamSynchronize(s);
-      return cuda_failed(e, "cudaEventRecord(upload ring)");
-    }
-    return THX_OK;
-  }
-  // host seconds spent waiting for space and copying into the ring
-  void times(double *wait_s, double *copy_s) {
-    std::lock_guard<std::mutex> lock(mu_);
-    *wait_s = wait_s_;
-    *copy_s = copy_s_;
-  }
-
- private:
-  bool fits(size_t bytes) const { return buf_ && ((bytes + 255) & ~size_t(255)) <= space_.capacity() / 2; }
-  std::mutex mu_;
-  double wait_s_ = 0.0, copy_s_ = 0.0;
-  unsigned char *buf_ = nullptr;
-  RingSpace space_;
-  std::deque<cudaEvent_t> busy_;  // one per live span, oldest first
-  std::vector<cudaEvent_t> spare_;
+  static void destroy(cudaEvent_t ev) { cudaEventDestroy(ev); }
+  static int record(cudaEvent_t ev, cudaStream_t s) { return status(cudaEventRecord(ev, s), "cudaEventRecord(upload ring)"); }
+  static int wait(cudaEvent_t ev) { return status(cudaEventSynchronize(ev), "cudaEventSynchronize(upload ring)"); }
+  static void drain(cudaStream_t s) { cudaStreamSynchronize(s); }
 };
+using HostRing = StagingRing<CudaStaging>;
 
 // Strides of the (possibly compressed) geometry arrays on the device.
 struct Layout {
