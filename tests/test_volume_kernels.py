@@ -136,3 +136,16 @@ def test_rate_over_its_state(cuda):
     u = to_dev(smooth_state(m, seed=5), torch.float64)
     ref = op.Mult(u, torch.empty_like(u))
     assert torch.equal(op.Mult(u, u), ref)
+
+
+@pytest.mark.parametrize("order,n", [(2, (4, 3, 4)), (4, (3, 4, 3)), (5, (3, 3, 3))])
+def test_viscous_rate_over_its_state(cuda, order, n):
+    """The same for Navier-Stokes: a mesh of the fused kernel falls back on the
+    gradient, face and volume kernels of the larger meshes, which an operator of
+    its size launches only here."""
+    import torch
+    m = box(3, order, n)
+    op = T.NSOperator(m, numerical_flux="ranocha", surface_flux="hll", mu=0.02)
+    u = to_dev(smooth_state(m, seed=5), torch.float64)
+    ref = op.Mult(u, torch.empty_like(u))
+    assert torch.equal(op.Mult(u, u), ref) and op.read_status() == 0

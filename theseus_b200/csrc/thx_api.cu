@@ -662,15 +662,18 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
     if ((st = dev_zero(h->isl_alpha, sizeof(double) * h->ne))) return st;
     h->islands = true;
   }
-  // kernel attributes (dynamic shared memory)
-  cudaError_t ce;
+  // Attributes (dynamic shared memory) of the kernels that run_rhs can launch;
+  // each also loads the kernel's image.  Meshes of the fused small-mesh kernel
+  // fall back on the separate ones for a result that overlaps its input.
+  const bool lines = h->small != 1, nodes = !h->aligned || h->small > 0;
+  cudaError_t ce = cudaSuccess;
   if (h->mixed) {
     VolArgs<float> va{};
     GradArgs<float> ga{};
-    ce = h->vol32(va, 0, 1);
+    if (lines) ce = h->vol32(va, 0, 1);
     if (ce == cudaSuccess && h->small) ce = h->small32(va, FaceArgs<float>{}, 0, 0, 1);
-    if (ce == cudaSuccess && h->ns) ce = h->grad32(ga, 0, 1);
-    if (ce == cudaSuccess && h->aligned) ce = h->gradl32(ga, nullptr, nullptr, 0, 1);
+    if (ce == cudaSuccess && h->ns && nodes) ce = h->grad32(ga, 0, 1);
+    if (ce == cudaSuccess && h->aligned && lines) ce = h->gradl32(ga, nullptr, nullptr, 0, 1);
     if (ce == cudaSuccess && h->blend) ce = h->fv32(va, 0, 1);
     if (ce == cudaSuccess && h->islands) {
       VolArgs<double> v64{};
@@ -680,10 +683,10 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
   } else {
     VolArgs<double> va{};
     GradArgs<double> ga{};
-    ce = h->vol64(va, 0, 1);
+    if (lines) ce = h->vol64(va, 0, 1);
     if (ce == cudaSuccess && h->small) ce = h->small64(va, FaceArgs<double>{}, 0, 0, 1);
-    if (ce == cudaSuccess && h->ns) ce = h->grad64(ga, 0, 1);
-    if (ce == cudaSuccess && h->aligned) ce = h->gradl64(ga, nullptr, nullptr, 0, 1);
+    if (ce == cudaSuccess && h->ns && nodes) ce = h->grad64(ga, 0, 1);
+    if (ce == cudaSuccess && h->aligned && lines) ce = h->gradl64(ga, nullptr, nullptr, 0, 1);
     if (ce == cudaSuccess && h->blend && h->fv64) ce = h->fv64(va, 0, 1);
   }
   if (ce != cudaSuccess) { cudaGetLastError(); return THX_ERR_CUDA; }
