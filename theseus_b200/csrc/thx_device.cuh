@@ -110,6 +110,9 @@ __device__ __forceinline__ double log_normal(double x) {
   const double a = kd * 0x1.62e42fefa3p-1, sum = a + f, dsum = (a - sum) + f;
   return sum - ((h - (__fma_rn(s, h + r * z, kd * 0x1.3de6af278ece6p-42) - dh)) - dsum);
 }
+// log(x) of any x.  Out of line: such arguments belong to states that are no
+// gas, and an inlined logarithm would lengthen every flux.
+static __device__ __noinline__ double log_any(double x) { return log(x); }
 // normal, positive and finite
 __device__ __forceinline__ bool is_normal_positive(double x) {
   return (unsigned)(__double2hiint(x) - 0x00100000) < 0x7FE00000u;
@@ -130,7 +133,7 @@ __device__ __forceinline__ double log_mean(double x, double y) {
     const double denom = 105.0 + u * (35.0 + u * (21.0 + 15.0 * u));
     return (x + y) * 52.5 / denom;
   }
-  return (y - x) / (is_normal_positive(xi) ? log_normal(xi) : log(xi));
+  return (y - x) / (is_normal_positive(xi) ? log_normal(xi) : log_any(xi));
 }
 // FP32 path: the same function with f = (xi-1)/(xi+1) = (y-x)/(y+x) formed
 // directly (one division; y-x is exact for near-equal arguments) and
