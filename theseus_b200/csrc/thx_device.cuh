@@ -413,27 +413,56 @@ __device__ __forceinline__ void vol_pirozzoli(const GasT<R> &g, const R *a, cons
   F[DIM + 1] = rho_mean * (h_mean + ke_mean) * vn;
 }
 
-// Central flux of HLL/LLF/Roe (include/HLLFlux.hpp:21-51): average of the
-// physical Euler fluxes contracted with the averaged metric.  qa/qb are the
-// conserved states, a/b the node data (aux = total enthalpy H).
+// Full conserved state from its stored form (adds qref in FP32).
 template <typename R, int DIM>
-__device__ __forceinline__ void vol_central(const R *qa, const R *qb, const R *a, const R *b,
-                                            const R *met, R *F) {
-  const R ia = fdiv(R(1), a[0]), ib = fdiv(R(1), b[0]);
+__device__ __forceinline__ void reconstruct(const GasT<R> &g, const R *raw, R *q) {
+#pragma unroll
+  for (int k = 0; k < DIM + 2; ++k) {
+    if constexpr (IsF32<R>::value) q[k] = g.qref[k] + raw[k];
+    else q[k] = raw[k];
+  }
+}
+
+// What the volume kernels keep of a node: node_prims' data less what the flux
+// does not read.  For the central flux the conserved state, 1/rho, the pressure
+// entering momentum fluxes and the total enthalpy.
+template <typename R, int DIM, int VOL>
+constexpr int node_fields() {
+  return VOL == VOL_CENTRAL ? DIM + 5 : nprim<R, DIM>() - (VOL == VOL_RANOCHA && !IsF32<R>::value ? 1 : 0);
+}
+template <typename R, int DIM, int VOL>
+__device__ __forceinline__ void pack_node(const GasT<R> &g, const R *raw, const R *pr, R *out) {
+  if constexpr (VOL == VOL_CENTRAL) {
+    reconstruct<R, DIM>(g, raw, out);
+    out[DIM + 2] = fdiv(R(1), pr[0]);
+    out[DIM + 3] = mom_p<R, DIM>(pr);
+    out[DIM + 4] = pr[DIM + 2];
+  } else {
+#pragma unroll
+    for (int k = 0; k < node_fields<R, DIM, VOL>(); ++k) out[k] = pr[k];
+  }
+}
+
+// Central flux of HLL/LLF/Roe (include/HLLFlux.hpp:21-51): average of the
+// physical Euler fluxes contracted with the averaged metric, from the nodes'
+// stored fields (pack_node).
+template <typename R, int DIM>
+__device__ __forceinline__ void vol_central(const R *a, const R *b, const R *met, R *F) {
+  const R ia = a[DIM + 2], ib = b[DIM + 2];
   R acc0 = R(0), accE = R(0);
   R accm[DIM];
 #pragma unroll
   for (int i = 0; i < DIM; ++i) accm[i] = R(0);
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
-    acc0 += R(0.5) * (qa[1 + d] + qb[1 + d]) * met[d];
+    acc0 += R(0.5) * (a[1 + d] + b[1 + d]) * met[d];
 #pragma unroll
     for (int i = 0; i < DIM; ++i) {
-      R fa = qa[1 + i] * qa[1 + d] * ia, fb = qb[1 + i] * qb[1 + d] * ib;
-      if (i == d) { fa += mom_p<R, DIM>(a); fb += mom_p<R, DIM>(b); }
+      R fa = a[1 + i] * a[1 + d] * ia, fb = b[1 + i] * b[1 + d] * ib;
+      if (i == d) { fa += a[DIM + 3]; fb += b[DIM + 3]; }
       accm[i] += R(0.5) * (fa + fb) * met[d];
     }
-    accE += R(0.5) * (qa[1 + d] * a[DIM + 2] + qb[1 + d] * b[DIM + 2]) * met[d];
+    accE += R(0.5) * (a[1 + d] * a[DIM + 4] + b[1 + d] * b[DIM + 4]) * met[d];
   }
   F[0] = acc0;
 #pragma unroll
@@ -478,16 +507,6 @@ __device__ __forceinline__ void make_fstate(const GasT<R> &g, const R *raw, FSta
     for (int k = 0; k < DIM + 2; ++k) { s.d[k] = raw[k]; s.q[k] = raw[k]; }
     s.p = pressure<R, DIM>(g, s.q);
     s.pp = s.p;
-  }
-}
-
-// Full conserved state from its stored form (adds qref in FP32).
-template <typename R, int DIM>
-__device__ __forceinline__ void reconstruct(const GasT<R> &g, const R *raw, R *q) {
-#pragma unroll
-  for (int k = 0; k < DIM + 2; ++k) {
-    if constexpr (IsF32<R>::value) q[k] = g.qref[k] + raw[k];
-    else q[k] = raw[k];
   }
 }
 

@@ -44,12 +44,11 @@ __host__ constexpr int small_mesh(int dim, int N, int ne, bool f32) {
 template <typename R, int DIM, int N, int VOL, bool FACES>
 struct SmallSmem {
   using S = Shape<DIM, N>;
-  static constexpr bool NEEDQ = VOL == VOL_CENTRAL;
-  static constexpr int PRIM = nprim<R, DIM>();
+  static constexpr int PRIM = node_fields<R, DIM, VOL>();
   static constexpr int FP = S::NEQ % 2 ? S::NEQ : S::NEQ + 1;  // stride of a pair's flux (odd: banks)
   static constexpr int PT = (DIM * S::PAIRS * 4 + 7) / 8 * 8;  // bytes of the pair table
   // values of R per element
-  static constexpr int ELEM = PRIM * S::ND + (NEEDQ ? S::NEQ * S::ND : 0) + DIM * S::PAIRS * FP +
+  static constexpr int ELEM = PRIM * S::ND + DIM * S::PAIRS * FP +
                               (FACES ? 2 * DIM * S::NEQ * S::NFP : 0);
   __host__ __device__ static constexpr size_t bytes(int epb) {
     return PT + sizeof(R) * (size_t)(S::OPS + epb * ELEM) + sizeof(int) * (size_t)epb * 2 * DIM;
@@ -75,8 +74,7 @@ __device__ __forceinline__ void small_body(const VolArgs<R> &a, const FaceArgs<R
   unsigned *sPT = reinterpret_cast<unsigned *>(smem_raw);  // [DIM][PAIRS] lower node | upper << 16
   R *sD = reinterpret_cast<R *>(smem_raw + M::PT);         // Dhat2
   R *sP = sD + S::OPS;                                     // [epb][PRIM][ND]
-  R *sQ = sP + epb * PRIM * ND;                            // [epb][NEQ][ND] if NEEDQ
-  R *sB = sQ + (M::NEEDQ ? epb * NEQ * ND : 0);            // [epb][DIM][PAIRS][FP] pair fluxes
+  R *sB = sP + epb * PRIM * ND;                            // [epb][DIM][PAIRS][FP] pair fluxes
   R *sF = sB + epb * DIM * PAIRS * M::FP;                  // [epb][2*DIM][NEQ][NFP] face fluxes
   int *sE = reinterpret_cast<int *>(sF + (FACES ? epb * 2 * DIM * NEQ * NFP : 0));  // [epb][2*DIM] elem_face
   const int tid = threadIdx.x;
@@ -111,16 +109,13 @@ __device__ __forceinline__ void small_body(const VolArgs<R> &a, const FaceArgs<R
   bool slow = false;
   for (int i = tid; i < cnt * ND; i += T) {
     const int el = i / ND, n = i - el * ND;
-    R q[NEQ], pr[PRIM];
+    R q[NEQ], pr[nprim<R, DIM>()], fl[PRIM];
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) q[k] = a.u[k * L + (long long)e0 * ND + i];
     node_prims<R, DIM, VOL>(a.gas, q, pr);
+    pack_node<R, DIM, VOL>(a.gas, q, pr, fl);
 #pragma unroll
-    for (int k = 0; k < PRIM; ++k) sP[(el * PRIM + k) * ND + n] = pr[k];
-    if (M::NEEDQ) {
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) sQ[(el * NEQ + k) * ND + n] = q[k];
-    }
+    for (int k = 0; k < PRIM; ++k) sP[(el * PRIM + k) * ND + n] = fl[k];
     if constexpr (!IsF32<R>::value) {
       if (!(pr[0] > R(0)) || !(pr[DIM + 1] > R(0))) atomicOr(a.status, STATUS_NONPOSITIVE);
       if constexpr (FASTABLE) slow = slow || !in_fast_range(pr[0]) || !in_fast_range(pr[DIM + 1]);
@@ -132,26 +127,19 @@ __device__ __forceinline__ void small_body(const VolArgs<R> &a, const FaceArgs<R
   for (int t = tid; t < cnt * DIM * PAIRS; t += T) {
     const int el = t / (DIM * PAIRS), p = t - el * (DIM * PAIRS), dir = p / PAIRS;
     const int na = (int)(sPT[p] & 0xffffu), nb = (int)(sPT[p] >> 16);
-    R A[PRIM], B[PRIM], QA[NEQ], QB[NEQ], met[DIM], F[NEQ];
+    R A[PRIM], B[PRIM], met[DIM], F[NEQ];
 #pragma unroll
     for (int k = 0; k < PRIM; ++k) {
       A[k] = sP[(el * PRIM + k) * ND + na];
       B[k] = sP[(el * PRIM + k) * ND + nb];
-    }
-    if (M::NEEDQ) {
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) {
-        QA[k] = sQ[(el * NEQ + k) * ND + na];
-        QB[k] = sQ[(el * NEQ + k) * ND + nb];
-      }
     }
     // one metric row per element: 0.5*(m+m) == m
     const R *m = a.met + (long long)(e0 + el) * a.met_es + dir * DIM;
 #pragma unroll
     for (int d = 0; d < DIM; ++d)
       met[d] = a.met_ns == 0 ? m[d] : R(0.5) * (m[(long long)na * a.met_ns + d] + m[(long long)nb * a.met_ns + d]);
-    if (FASTABLE && slow) pair_flux<R, DIM, VOL, false, LM_BRANCH>(a.gas, A, B, QA, QB, met, F);
-    else pair_flux<R, DIM, VOL, FASTABLE, LM_BRANCH>(a.gas, A, B, QA, QB, met, F);
+    if (FASTABLE && slow) pair_flux<R, DIM, VOL, false, LM_BRANCH>(a.gas, A, B, met, F);
+    else pair_flux<R, DIM, VOL, FASTABLE, LM_BRANCH>(a.gas, A, B, met, F);
 #pragma unroll
     for (int k = 0; k < NEQ; ++k) sB[t * M::FP + k] = F[k];
   }

@@ -45,10 +45,8 @@ constexpr int kLineThreads = 128;
 template <typename R, int DIM, int N, int VOL, int T, int EPBX = 0>
 struct LineSmem {
   using S = LineShape<DIM, N, T, EPBX>;
-  static constexpr bool NEEDQ = VOL == VOL_CENTRAL;
-  // the Ranocha flux reads no auxiliary (the last field of the FP64 layout)
-  static constexpr int PRIM = nprim<R, DIM>() - ((VOL == VOL_RANOCHA && !IsF32<R>::value) ? 1 : 0);
-  static constexpr int FIELDS = PRIM + S::NEQ + (NEEDQ ? S::NEQ : 0);
+  static constexpr int PRIM = node_fields<R, DIM, VOL>();
+  static constexpr int FIELDS = PRIM + S::NEQ;
   static constexpr int OPS = (N * N + 1) / 2 * 2;
   static constexpr int MET = (S::EPB * DIM * DIM + 1) / 2 * 2;  // one metric per element
   static constexpr size_t bytes() {
@@ -163,19 +161,13 @@ __device__ __forceinline__ void pair_ranocha(const GasT<double> &g, const double
 // The two-point flux of a pair.  SHARED: with the shared reciprocals (FP64;
 // every density and pressure in their range).
 template <typename R, int DIM, int VOL, bool SHARED, int MODE>
-__device__ __forceinline__ void pair_flux(const GasT<R> &g, const R *A, const R *B, const R *qa, const R *qb,
-                                          const R *met, R *F) {
+__device__ __forceinline__ void pair_flux(const GasT<R> &g, const R *A, const R *B, const R *met, R *F) {
   if constexpr (SHARED && VOL == VOL_CHANDRASHEKAR) pair_chandrashekar<DIM, MODE>(g, A, B, met, F);
   else if constexpr (SHARED && VOL == VOL_RANOCHA) pair_ranocha<DIM, MODE>(g, A, B, met, F);
   else if constexpr (VOL == VOL_CHANDRASHEKAR) vol_chandrashekar<R, DIM, MODE>(g, A, B, met, F);
   else if constexpr (VOL == VOL_RANOCHA) vol_ranocha<R, DIM, MODE>(g, A, B, met, F);
   else if constexpr (VOL == VOL_PIROZZOLI) vol_pirozzoli<R, DIM>(g, A, B, met, F);
-  else {
-    R ca[DIM + 2], cb[DIM + 2];
-    reconstruct<R, DIM>(g, qa, ca);
-    reconstruct<R, DIM>(g, qb, cb);
-    vol_central<R, DIM>(ca, cb, A, B, met, F);
-  }
+  else vol_central<R, DIM>(A, B, met, F);
 }
 
 // Whether every logarithmic mean between the nodes of a line takes its
@@ -405,8 +397,7 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
   R *sM = sD + M::OPS;                      // [EPB][DIM][DIM] metric rows (one per element)
   R *sP = sM + M::MET;                      // [PRIM][EPB][NDP] node data
   R *sR = sP + PRIM * FS;                   // [NEQ][EPB][NDP] sums of the directions so far
-  R *sQ = sR + NEQ * FS;                    // [NEQ][EPB][NDP] state (central flux)
-  int *sF = reinterpret_cast<int *>(sQ + (M::NEEDQ ? NEQ * FS : 0));  // [EPB][2*DIM] elem_face
+  int *sF = reinterpret_cast<int *>(sR + NEQ * FS);  // [EPB][2*DIM] elem_face
   const int tid = threadIdx.x;
   const int e0 = block * EPB;
   const long long L = (long long)a.ne * ND;
@@ -432,17 +423,14 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
     const int i = tid + it * T;
-    R pr[nprim<R, DIM>()];
+    R pr[nprim<R, DIM>()], fl[PRIM];
     const R *q = qn[it];
     if (i >= nodes) continue;
     node_prims<R, DIM, VOL>(a.gas, q, pr);
+    pack_node<R, DIM, VOL>(a.gas, q, pr, fl);
     const int pn = i + (N % 2 ? 0 : i / N);
 #pragma unroll
-    for (int k = 0; k < PRIM; ++k) sP[k * FS + pn] = pr[k];
-    if (M::NEEDQ) {
-#pragma unroll
-      for (int k = 0; k < NEQ; ++k) sQ[k * FS + pn] = q[k];
-    }
+    for (int k = 0; k < PRIM; ++k) sP[k * FS + pn] = fl[k];
     if constexpr (!IsF32<R>::value) {
       // FP64 path: positivity of the state read here.  FP32-mixed: checked
       // on the FP64 master state instead (to_working, the RK stage epilogue)
@@ -490,13 +478,9 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
 #pragma unroll
       for (int d = 0; d < DIM; ++d) met[d] = sM[(el * DIM + dir) * DIM + d];
     }
-    auto load = [&](int s, R *P, R *Q) {
+    auto load = [&](int s, R *P) {
 #pragma unroll
       for (int k = 0; k < PRIM; ++k) P[k] = sP[k * FS + s];
-      if (M::NEEDQ) {
-#pragma unroll
-        for (int k = 0; k < NEQ; ++k) Q[k] = sQ[k * FS + s];
-      }
     };
     // averaged metric row of a pair (one row per element: 0.5*(m+m) == m)
     auto pair_met = [&](int i, int j, R *m) {
@@ -520,13 +504,13 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
         for (int k = 0; k < NEQ; ++k) acc[i][k] = dir == 0 ? R(0) : sR[k * FS + base + i * stride];
 #pragma unroll
       for (int i = 0; i < N - 1; ++i) {
-        R A[nprim<R, DIM>()], QA[NEQ];
-        load(base + i * stride, A, QA);
+        R A[PRIM];
+        load(base + i * stride, A);
 #pragma unroll
         for (int j = i + 1; j < N; ++j) {
-          R B[nprim<R, DIM>()], QB[NEQ], F[NEQ];
-          load(base + j * stride, B, QB);
-          pair_flux<R, DIM, VOL, FASTABLE, LM_SERIES>(a.gas, A, B, QA, QB, met, F);
+          R B[PRIM], F[NEQ];
+          load(base + j * stride, B);
+          pair_flux<R, DIM, VOL, FASTABLE, LM_SERIES>(a.gas, A, B, met, F);
           const R ci = sD[i * N + j], cj = sD[j * N + i];
 #pragma unroll
           for (int k = 0; k < NEQ; ++k) {
@@ -551,18 +535,18 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
 #pragma unroll 1
       for (int i = 0; i < N - 1; ++i) {
         const int si = base + i * stride;
-        R A[nprim<R, DIM>()], QA[NEQ], sum[NEQ];
-        load(si, A, QA);
+        R A[PRIM], sum[NEQ];
+        load(si, A);
 #pragma unroll
         for (int k = 0; k < NEQ; ++k) sum[k] = sR[k * FS + si];
         auto pairs = [&](auto shared) {
 #pragma unroll 1
           for (int j = i + 1; j < N; ++j) {
             const int sj = base + j * stride;
-            R B[nprim<R, DIM>()], QB[NEQ], m[DIM], F[NEQ];
-            load(sj, B, QB);
+            R B[PRIM], m[DIM], F[NEQ];
+            load(sj, B);
             pair_met(i, j, m);
-            pair_flux<R, DIM, VOL, decltype(shared)::value, LM_BRANCH>(a.gas, A, B, QA, QB, m, F);
+            pair_flux<R, DIM, VOL, decltype(shared)::value, LM_BRANCH>(a.gas, A, B, m, F);
             const R ci = sD[i * N + j], cj = sD[j * N + i];
 #pragma unroll
             for (int k = 0; k < NEQ; ++k) {
