@@ -211,3 +211,28 @@ def test_serving_loop_small_stream(cuda):
         assert field_errors(r, alone(c, "fp32"), 2).max() <= 1e-5
         assert field_errors(r, alone(c, "fp64"), 2).max() <= 1e-5
         assert np.all(np.isfinite(r))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_engine_metric_per_node(cuda, precision):
+    """Meshes whose metric varies within the element beside boxes of the same
+    order: each case equals its one-case run."""
+    from _helpers import random_geometry
+    batch = []
+    for i, (dim, order, n, viscous) in enumerate([(2, 2, (7, 6), False), (2, 3, (5, 6), True), (3, 4, (2, 3, 2), True),
+                                                  (3, 5, (2, 2, 2), False)]):
+        for curved in (True, False):
+            c = vortex_case(dim, order, n, viscous, 12, seed=20 + i)
+            if curved:
+                c.mesh = random_geometry(c.mesh, seed=i, amp=0.01)
+            batch.append(c)
+    eng = BatchEngine(precision=precision, steps_per_launch=4, **FLUX)
+    out = run_engine(eng, batch)
+    assert len(eng.groups()) == len(batch)
+    eng.close()
+    for c, got in zip(batch, out):
+        ref = alone(c, precision)
+        if precision == "fp64":
+            assert np.array_equal(got, ref)
+        else:
+            assert field_errors(got, ref, c.mesh.dim).max() <= 1e-5

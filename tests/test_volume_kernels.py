@@ -149,3 +149,17 @@ def test_viscous_rate_over_its_state(cuda, order, n):
     u = to_dev(smooth_state(m, seed=5), torch.float64)
     ref = op.Mult(u, torch.empty_like(u))
     assert torch.equal(op.Mult(u, u), ref) and op.read_status() == 0
+
+
+@pytest.mark.parametrize("dim,order", sorted(SIZES))
+def test_metric_per_node(cuda, dim, order):
+    """Metrics that vary within the element, by the line kernel, on both of its
+    paths; one of all elements alike too (an element stride of zero)."""
+    m = random_geometry(box(dim, order, SIZES[dim, order][2]), seed=order)
+    nearly = cases.perturbed_uniform(m.state_shape(), dim, seed=3, amp=1e-3)
+    for vol, surf, ns in (("chandrashekar", "roe", False), ("ranocha", "hll", True), ("hll", "llf", False)):
+        kw = dict(numerical_flux=vol, surface_flux=surf, **({"mu": 0.03} if ns else {}))
+        compare(m, smooth_state(m, seed=order), ns, **kw)
+        compare(m, nearly, ns, **kw)
+    m.metric[...] = m.metric[:1]
+    compare(m, smooth_state(m, seed=order), True, numerical_flux="ranocha", surface_flux="hll", mu=0.03)

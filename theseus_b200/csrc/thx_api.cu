@@ -204,16 +204,17 @@ bool pick_order_kernels(thx_operator_s *h, int vk) {
 #define THX_PICK(P, D, NN)                                                  \
   if (h->dim == D && h->N == NN) {                                          \
     auto k = order_kernels_##P##_##D##_##NN();                              \
-    const bool tma = h->cfg.volume_staging == 1 && !bl;                    \
+    const bool nodal = h->lay.met_ns != 0;                                  \
+    const bool tma = h->cfg.volume_staging == 1 && !bl && !nodal;           \
     if (P == 0) {                                                           \
-      h->vol64 = reinterpret_cast<VolLaunch<double>>(tma ? k.vol_tma[vk] : k.vol[vk]); \
+      h->vol64 = reinterpret_cast<VolLaunch<double>>(tma ? k.vol_tma[vk] : k.vol[vk][nodal]); \
       h->small64 = reinterpret_cast<SmallLaunch<double>>(k.small[vk][h->small > 1]); \
       h->grad64 = reinterpret_cast<GradLaunch<double>>(k.grad);             \
       h->gradl64 = reinterpret_cast<GradLineLaunch<double>>(k.grad_line);   \
       h->blend64 = reinterpret_cast<BlendLaunch<double>>(k.blend);          \
       h->fv64 = reinterpret_cast<VolLaunch<double>>(k.fv);                  \
     } else {                                                                \
-      h->vol32 = reinterpret_cast<VolLaunch<float>>(tma ? k.vol_tma[vk] : k.vol[vk]); \
+      h->vol32 = reinterpret_cast<VolLaunch<float>>(tma ? k.vol_tma[vk] : k.vol[vk][nodal]); \
       h->small32 = reinterpret_cast<SmallLaunch<float>>(k.small[vk][h->small > 1]);  \
       h->grad32 = reinterpret_cast<GradLaunch<float>>(k.grad);              \
       h->gradl32 = reinterpret_cast<GradLineLaunch<float>>(k.grad_line);    \
@@ -468,7 +469,21 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
   if (!donor) {
   pack_strided(g->jac, h->ne, nd, 1, full, tmp, h->lay.jac_es, h->lay.jac_ns);
   if ((st = upload_both(tmp, &h->jac64, &h->jac32, w32, A))) return st;
-  pack_strided(g->metric, h->ne, nd, MB, full, tmp, h->lay.met_es, h->lay.met_ns);
+  long long met_ns;
+  pack_strided(g->metric, h->ne, nd, MB, full, tmp, h->lay.met_es, met_ns);
+  if (met_ns != 0) {
+    // varying within the element: each element's block by components, so that
+    // neighbouring threads, which have neighbouring nodes, read neighbouring
+    // values
+    std::vector<double> block((size_t)MB * nd);
+    for (size_t o = 0; o < tmp.size(); o += block.size()) {
+      for (int i = 0; i < nd; ++i)
+        for (int k = 0; k < MB; ++k) block[(size_t)k * nd + i] = tmp[o + (size_t)i * MB + k];
+      std::copy(block.begin(), block.end(), tmp.begin() + o);
+    }
+    h->lay.met_ns = 1;
+    h->lay.met_cs = nd;
+  }
   if ((st = upload_both(tmp, &h->met64, &h->met32, w32, A))) return st;
   pack_strided(g->face_normal, h->nf, nfp, dim, full, tmp, h->lay.n_fs, h->lay.n_ps);
   // normals are indexed as (f*n_fs + fp*n_ps)*DIM: convert block strides to point units
@@ -545,6 +560,8 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
     if ((st = upload_both(ops, &h->ops64, &h->ops32, w32, A))) return st;
     if ((st = upload_both(D, &h->D64, &h->D32, w32, A))) return st;
   }
+  // the volume kernel depends on the metric's layout, known only now
+  if (!h->lte) pick_order_kernels(h, vk);
   // scratch
   const size_t fsz = (size_t)(h->nf + h->nbf) * h->neq * nfp;
   // the line volume kernel takes the viscous divergence from the gradient kernel
@@ -629,7 +646,7 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
 #define THX_PICK_ISL(P, D, NN)                                   \
     if (h->dim == D && h->N == NN) {                             \
       auto k = order_kernels_0_##D##_##NN();                     \
-      h->isl_vol = k.voll[vk];                                   \
+      h->isl_vol = k.voll[vk][h->lay.met_ns != 0];                                   \
       h->isl_fv = k.fvl;                                         \
       h->isl_blend = k.blendl;                                   \
       found = true;                                              \
@@ -693,7 +710,7 @@ int create_impl(const thx_geometry *g, const thx_config *cfg, thx_operator_s *h,
   char buf[512];
   std::snprintf(buf, sizeof(buf),
                 "dim=%d p=%d ne=%d nf=%d flow=%s gas=%s vol=%d surf=%d fv=%d blend=%d prec=%s "
-                "layout jac(%lld,%lld) met(%lld,%lld) nrm(%lld,%lld) w(%lld,%lld) sub(%lld)",
+                "layout jac(%lld,%lld) met(%lld,%d) nrm(%lld,%lld) w(%lld,%lld) sub(%lld)",
                 dim, h->order, h->ne, h->nf, h->ns ? "ns" : "euler", h->lte ? "lte" : "ideal",
                 cfg->volume_flux, cfg->surface_flux, cfg->fv_flux, cfg->blending,
                 h->mixed ? "fp32-mixed" : "fp64",
@@ -747,7 +764,7 @@ void op_args(thx_operator_s *h, const R *u, R *du, int stage, double dt, double 
   ga = GradArgs<R>{};
   ga.u = u; ga.vflux = vfl; ga.vdiv = reinterpret_cast<R *>(h->vdiv); ga.ne = h->ne;
   ga.jac = G.jac; ga.jac_es = h->lay.jac_es; ga.jac_ns = h->lay.jac_ns;
-  ga.met = G.met; ga.met_es = h->lay.met_es; ga.met_ns = h->lay.met_ns;
+  ga.met = G.met; ga.met_es = h->lay.met_es; ga.met_ns = h->lay.met_ns; ga.met_cs = h->lay.met_cs;
   ga.elem_face = h->elem_face; ga.face_elem = h->face_elem; ga.face_lface = h->face_lface;
   ga.normal = G.nrm; ga.n_fs = h->lay.n_fs; ga.n_ps = h->lay.n_ps;
   ga.wm = G.wm; ga.wp = G.wp; ga.w_fs = h->lay.w_fs; ga.w_ps = h->lay.w_ps;
@@ -770,7 +787,7 @@ void op_args(thx_operator_s *h, const R *u, R *du, int stage, double dt, double 
   va = VolArgs<R>{};
   va.u = u; va.du = du; va.ne = h->ne;
   va.jac = G.jac; va.jac_es = h->lay.jac_es; va.jac_ns = h->lay.jac_ns;
-  va.met = G.met; va.met_es = h->lay.met_es; va.met_ns = h->lay.met_ns;
+  va.met = G.met; va.met_es = h->lay.met_es; va.met_ns = h->lay.met_ns; va.met_cs = h->lay.met_cs;
   va.elem_face = h->elem_face; va.fstar = fst;
   va.wm = G.wm; va.wp = G.wp; va.w_fs = h->lay.w_fs; va.w_ps = h->lay.w_ps;
   va.vflux = vfl;
@@ -1041,7 +1058,7 @@ int stability_rates(thx_operator_s *h, const double *u, cudaStream_t s) {
   StabArgs a;
   a.u = u; a.ne = h->ne; a.N = h->N;
   a.jac = h->jac64; a.jac_es = h->lay.jac_es; a.jac_ns = h->lay.jac_ns;
-  a.met = h->met64; a.met_es = h->lay.met_es; a.met_ns = h->lay.met_ns;
+  a.met = h->met64; a.met_es = h->lay.met_es; a.met_ns = h->lay.met_ns; a.met_cs = h->lay.met_cs;
   a.face_elem = h->face_elem; a.face_lface = h->face_lface; a.nf = h->nf;
   a.normal = h->nrm64; a.n_fs = h->lay.n_fs; a.n_ps = h->lay.n_ps;
   a.wm = h->wm64; a.wp = h->wp64; a.w_fs = h->lay.w_fs; a.w_ps = h->lay.w_ps;

@@ -88,7 +88,7 @@ struct EngineBase {
 template <typename R>
 struct Group {
   int dim = 0, N = 0;
-  bool ns = false;
+  bool ns = false, nodal = false;
   int epb = 1, nfp = 1;  // epb: elements per CTA of the current tables
   int epb_full = 1, epb_half = 0;
   std::vector<EngineCase *> cases;
@@ -485,7 +485,7 @@ class Engine final : public EngineBase {
   }
 
  private:
-  using Key = std::tuple<int, int, bool>;
+  using Key = std::tuple<int, int, bool, bool>;
 
   struct Bounce {
     cudaStream_t stream = nullptr;  // the copies' stream, kept with the buffer
@@ -543,7 +543,9 @@ class Engine final : public EngineBase {
   }
 
   int group_for(thx_operator_s *h, Group<R> **out) {
-    const Key key(h->dim, h->N, h->ns);
+    // meshes whose metric varies within the element run other kernels
+    const bool nodal = h->lay.met_ns != 0;
+    const Key key(h->dim, h->N, h->ns, nodal);
     auto it = groups_.find(key);
     if (it != groups_.end()) {
       *out = it->second.get();
@@ -553,6 +555,7 @@ class Engine final : public EngineBase {
     G->dim = h->dim;
     G->N = h->N;
     G->ns = h->ns;
+    G->nodal = nodal;
     G->nfp = h->nfp;
     const int vk = (cfg_.volume_flux == THX_FLUX_CHANDRASHEKAR) ? VOL_CHANDRASHEKAR
                  : (cfg_.volume_flux == THX_FLUX_RANOCHA)     ? VOL_RANOCHA
@@ -940,11 +943,11 @@ void Engine<double>::pick_kernels(Group<double> &G, int vk, int ns) {
 #define THX_PICKB(P, D, NN)                                 \
   if (G.dim == D && G.N == NN) {                            \
     const OrderKernels0 k = order_kernels_##P##_##D##_##NN(); \
-    G.volb = k.volb[vk];                                \
+    G.volb = k.volb[vk][G.nodal];                           \
     G.gradb = k.gradb;                                      \
     G.epb_full = k.epb;                                     \
     G.epb_half = k.epb_half;                                \
-    G.volb_half = k.volb_half[vk];                      \
+    G.volb_half = k.volb_half[vk][G.nodal];                 \
     G.gradb_half = k.gradb_half;                            \
   }
   THX_FOR_ORDERS(THX_PICKB, 0, 2)
@@ -959,11 +962,11 @@ void Engine<float>::pick_kernels(Group<float> &G, int vk, int ns) {
 #define THX_PICKB(P, D, NN)                                 \
   if (G.dim == D && G.N == NN) {                            \
     const OrderKernels1 k = order_kernels_##P##_##D##_##NN(); \
-    G.volb = k.volb[vk];                                \
+    G.volb = k.volb[vk][G.nodal];                           \
     G.gradb = k.gradb;                                      \
     G.epb_full = k.epb;                                     \
     G.epb_half = k.epb_half;                                \
-    G.volb_half = k.volb_half[vk];                      \
+    G.volb_half = k.volb_half[vk][G.nodal];                 \
     G.gradb_half = k.gradb_half;                            \
   }
   THX_FOR_ORDERS(THX_PICKB, 1, 2)

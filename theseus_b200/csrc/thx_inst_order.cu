@@ -20,11 +20,13 @@ THX_TYPE(THX_PREC) THX_NAME(THX_PREC, THX_DIM, THX_N)() {
   using R = THX_RT(THX_PREC);
   THX_TYPE(THX_PREC) k;
 #define THX_SETV(V)                                           \
-  k.vol[V] = &launch_volume_line<R, THX_DIM, THX_N, V>;        \
+  k.vol[V][0] = &launch_volume_line<R, THX_DIM, THX_N, V, false>; \
+  k.vol[V][1] = &launch_volume_line<R, THX_DIM, THX_N, V, true>;  \
   k.small[V][0] = &launch_volume_small<R, THX_DIM, THX_N, V, false>; \
   k.small[V][1] = &launch_volume_small<R, THX_DIM, THX_N, V, true>;  \
   k.vol_tma[V] = &launch_volume_tma<R, THX_DIM, THX_N, V>;     \
-  k.volb[V] = &launch_volume_batched<R, THX_DIM, THX_N, V>;
+  k.volb[V][0] = &launch_volume_batched<R, THX_DIM, THX_N, V, false>; \
+  k.volb[V][1] = &launch_volume_batched<R, THX_DIM, THX_N, V, true>;
   THX_SETV(VOL_CHANDRASHEKAR)
   THX_SETV(VOL_RANOCHA)
   THX_SETV(VOL_PIROZZOLI)
@@ -41,7 +43,8 @@ THX_TYPE(THX_PREC) THX_NAME(THX_PREC, THX_DIM, THX_N)() {
   k.gradb = &launch_grad_batched<R, THX_DIM, THX_N>;
   k.epb = Shape<THX_DIM, THX_N>::EPB;
   k.epb_half = half_epb<THX_DIM, THX_N>();
-  for (auto &v : k.volb_half) v = nullptr;
+  for (auto &row : k.volb_half)
+    for (auto &v : row) v = nullptr;
   k.gradb_half = nullptr;
   if constexpr (half_epb<THX_DIM, THX_N>() > 0) {
     constexpr int H = half_epb<THX_DIM, THX_N>();
@@ -49,9 +52,11 @@ THX_TYPE(THX_PREC) THX_NAME(THX_PREC, THX_DIM, THX_N)() {
     // multiply-adds differently in the two, and a case's result must not depend
     // on what the tuner finds for the cases beside it.
 #if THX_PREC == 0
-#define THX_SETH(V) k.volb_half[V] = &launch_volume_batched_pairs<R, THX_DIM, THX_N, V, H>;
+#define THX_SETH(V) k.volb_half[V][0] = k.volb_half[V][1] = &launch_volume_batched_pairs<R, THX_DIM, THX_N, V, H>;
 #else
-#define THX_SETH(V) k.volb_half[V] = &launch_volume_batched<R, THX_DIM, THX_N, V, H>;
+#define THX_SETH(V)                                                          \
+  k.volb_half[V][0] = &launch_volume_batched<R, THX_DIM, THX_N, V, false, H>; \
+  k.volb_half[V][1] = &launch_volume_batched<R, THX_DIM, THX_N, V, true, H>;
 #endif
     THX_SETH(VOL_CHANDRASHEKAR)
     THX_SETH(VOL_RANOCHA)
@@ -61,14 +66,19 @@ THX_TYPE(THX_PREC) THX_NAME(THX_PREC, THX_DIM, THX_N)() {
     k.gradb_half = &launch_grad_batched<R, THX_DIM, THX_N, H>;
   }
 #if THX_PREC == 0
-  k.voll[VOL_CHANDRASHEKAR] = &launch_volume_list<R, THX_DIM, THX_N, VOL_CHANDRASHEKAR>;
-  k.voll[VOL_RANOCHA] = &launch_volume_list<R, THX_DIM, THX_N, VOL_RANOCHA>;
-  k.voll[VOL_PIROZZOLI] = &launch_volume_list<R, THX_DIM, THX_N, VOL_PIROZZOLI>;
-  k.voll[VOL_CENTRAL] = &launch_volume_list<R, THX_DIM, THX_N, VOL_CENTRAL>;
+#define THX_SETL(V)                                                  \
+  k.voll[V][0] = &launch_volume_list<R, THX_DIM, THX_N, V, false>; \
+  k.voll[V][1] = &launch_volume_list<R, THX_DIM, THX_N, V, true>;
+  THX_SETL(VOL_CHANDRASHEKAR)
+  THX_SETL(VOL_RANOCHA)
+  THX_SETL(VOL_PIROZZOLI)
+  THX_SETL(VOL_CENTRAL)
+#undef THX_SETL
   k.fvl = &launch_fv_list<R, THX_DIM, THX_N>;
   k.blendl = &launch_blend_list<R, THX_DIM, THX_N>;
 #else
-  for (auto &v : k.voll) v = nullptr;
+  for (auto &row : k.voll)
+    for (auto &v : row) v = nullptr;
   k.fvl = nullptr;
   k.blendl = nullptr;
 #endif

@@ -5,9 +5,11 @@
 //   viscous flux     fv[d][eq-1][elem][node] (physical viscous flux, NS only;
 //                    its mass row is identically zero and is not stored)
 //   face fluxes      fs[face][eq][fp]       (unweighted F*, inviscid minus viscous)
-//   geometry         jac[e*jac_es + n*jac_ns], metric block of DIM*DIM per node
-//                    at met[e*met_es + n*met_ns]; strides are 0 where the host
-//                    found the factor constant (exactly) over nodes/elements.
+//   geometry         jac[e*jac_es + n*jac_ns], metric component k of DIM*DIM per
+//                    node at met[e*met_es + n*met_ns + k*met_cs]; strides are 0
+//                    where the host found the factor constant (exactly) over
+//                    nodes/elements.  A metric that varies within the element is
+//                    stored [elem][component][node] (met_ns = 1).
 //
 // Kernel structure per right-hand side:
 //   NS only : a gradient kernel: element-local BR1 gradient of entropy
@@ -145,7 +147,8 @@ struct VolArgs {
   const R *jac;
   long long jac_es, jac_ns;
   const R *met;
-  long long met_es, met_ns;
+  long long met_es;
+  int met_ns, met_cs;
   const int *elem_face;   // [e][2*DIM] = 2*face + side
   const R *fstar;         // [f][eq][fp]
   const R *wm, *wp;       // lift weights
@@ -276,9 +279,9 @@ __device__ __forceinline__ void lte_volume_body(const VolArgs<double> &a, const 
     for (int k = 0; k < NPRIM; ++k) sPrim[(el * NPRIM + k) * ND + n] = pr[k];
     if (!sv.valid || !(q[0] > 0.0)) atomicOr(a.status, STATUS_EOS);
     if (mns != 0 || n == 0) {
-      const R *mp = a.met + (long long)e * a.met_es + (long long)n * a.met_ns;
+      const R *mp = a.met + (long long)e * a.met_es + n * a.met_ns;
 #pragma unroll
-      for (int k = 0; k < MB; ++k) sMet[el * mbk + n * mns + k] = mp[k];
+      for (int k = 0; k < MB; ++k) sMet[el * mbk + n * mns + k] = mp[k * a.met_cs];
     }
   }
   __syncthreads();
@@ -827,7 +830,8 @@ struct GradArgs {
   const R *jac;
   long long jac_es, jac_ns;
   const R *met;
-  long long met_es, met_ns;
+  long long met_es;
+  int met_ns, met_cs;
   const int *elem_face, *face_elem, *face_lface;
   const R *normal;
   long long n_fs, n_ps;
@@ -866,19 +870,19 @@ __host__ __device__ constexpr size_t max_of(size_t x, size_t y) { return x > y ?
 // Every thread of the CTA calls it; the region sFv may be in use before.
 template <typename R, int DIM, int N, int EPBX = 0>
 __device__ __forceinline__ void viscous_divergence(const GradArgs<R> &a, const R *sDh, R *sFv, const R *vf,
-                                                   const R *row, const int el, const int n, const int e,
-                                                   const bool active) {
+                                                   const int el, const int n, const int e, const bool active) {
   using S = Shape<DIM, N, EPBX>;
   constexpr int ND = S::ND, NV = S::NEQ - 1;
   __syncthreads();
   if (active) {
+    const R *row = a.met + (long long)e * a.met_es + n * a.met_ns;
 #pragma unroll
     for (int dir = 0; dir < DIM; ++dir)
 #pragma unroll
       for (int k = 0; k < NV; ++k) {
         R f = R(0);
 #pragma unroll
-        for (int pd = 0; pd < DIM; ++pd) f += row[dir * DIM + pd] * vf[pd * NV + k];
+        for (int pd = 0; pd < DIM; ++pd) f += row[(dir * DIM + pd) * a.met_cs] * vf[pd * NV + k];
         sFv[((el * DIM + dir) * NV + k) * ND + n] = f;
       }
   }
@@ -1050,10 +1054,10 @@ __device__ __forceinline__ void grad_body(const GradArgs<R> &a, const int block)
     }
   }
   const R invJ = R(1) / a.jac[(long long)e * a.jac_es + (long long)n * a.jac_ns];
-  const R *adj = a.met + (long long)e * a.met_es + (long long)n * a.met_ns;
+  const R *adj = a.met + (long long)e * a.met_es + n * a.met_ns;
   R adjr[DIM * DIM];
 #pragma unroll
-  for (int k = 0; k < DIM * DIM; ++k) adjr[k] = adj[k];
+  for (int k = 0; k < DIM * DIM; ++k) adjr[k] = adj[k * a.met_cs];
   R g[DIM][NEQ];
 #pragma unroll
   for (int cc = 0; cc < DIM; ++cc)
@@ -1185,8 +1189,7 @@ __device__ __forceinline__ void grad_body(const GradArgs<R> &a, const int block)
   };
   if (active) node();
   if (a.vdiv)
-    viscous_divergence<R, DIM, N, EPBX>(a, sDh, sS, vfs, a.met + (long long)e * a.met_es + (long long)n * a.met_ns,
-                                        el, n, e, active);
+    viscous_divergence<R, DIM, N, EPBX>(a, sDh, sS, vfs, el, n, e, active);
 }
 
 // Shared memory of the gradient kernel that reads precomputed entropy
@@ -1311,7 +1314,7 @@ __device__ __forceinline__ void grad_body_sv(const GradArgs<R> &a, const int blo
   auto node = [&]() {
   int c[3];
   node_coords<DIM, N>(n, c);
-  const R *adj = a.met + (long long)e * a.met_es + (long long)n * a.met_ns;
+  const R *adj = a.met + (long long)e * a.met_es + n * a.met_ns;
   // physical gradient: sum over directions of D-derivative x adjugate row
   R g[DIM][NEQ];
 #pragma unroll
@@ -1332,7 +1335,7 @@ __device__ __forceinline__ void grad_body_sv(const GradArgs<R> &a, const int blo
     }
 #pragma unroll
     for (int cc = 0; cc < DIM; ++cc) {
-      const R ar = adj[dir * DIM + cc];
+      const R ar = adj[(dir * DIM + cc) * a.met_cs];
 #pragma unroll
       for (int k = 0; k < NEQ; ++k) {
         if (dir == 0) g[cc][k] = dr[k] * ar;
@@ -1437,8 +1440,7 @@ __device__ __forceinline__ void grad_body_sv(const GradArgs<R> &a, const int blo
   if (active) node();
   // the staged variables, state and lift factors are no longer needed
   if (a.vdiv)
-    viscous_divergence<R, DIM, N>(a, sDh, sS, vfs, a.met + (long long)e * a.met_es + (long long)n * a.met_ns, el, n,
-                                  e, active);
+    viscous_divergence<R, DIM, N>(a, sDh, sS, vfs, el, n, e, active);
 }
 
 }  // namespace thx
@@ -1713,7 +1715,8 @@ struct StabArgs {
   const double *jac;
   long long jac_es, jac_ns;
   const double *met;
-  long long met_es, met_ns;
+  long long met_es;
+  int met_ns, met_cs;
   const int *face_elem, *face_lface;
   int nf;
   const double *normal;
@@ -1760,7 +1763,7 @@ __global__ void stability_kernel(const StabArgs a) {
         double vdm = 0.0, mn2 = 0.0;
 #pragma unroll
         for (int pd = 0; pd < DIM; ++pd) {
-          const double v = M[rd * DIM + pd];
+          const double v = M[(rd * DIM + pd) * a.met_cs];
           vdm += (q[1 + pd] / q[0]) * v;
           mn2 += v * v;
         }
@@ -1805,7 +1808,10 @@ __global__ void stability_kernel(const StabArgs a) {
           for (int rd = 0; rd < DIM; ++rd) {
             double mn2 = 0.0;
 #pragma unroll
-            for (int pd = 0; pd < DIM; ++pd) mn2 += M[rd * DIM + pd] * M[rd * DIM + pd];
+            for (int pd = 0; pd < DIM; ++pd) {
+              const double v = M[(rd * DIM + pd) * a.met_cs];
+              mn2 += v * v;
+            }
             mss += mn2 * ij * ij;
           }
           const double mu = viscosity<double, DIM>(a.gas, qe);
@@ -1904,9 +1910,9 @@ template <typename R, int DIM, int N, int EPBX>
 constexpr int line_batch_threads() {
   return line_threads<DIM, N, Shape<DIM, N, EPBX>::EPB>();
 }
-template <typename R, int DIM, int N, int VOL, int EPBX = 0>
+template <typename R, int DIM, int N, int VOL, bool NODAL, int EPBX = 0>
 __global__ void __launch_bounds__((line_batch_threads<R, DIM, N, EPBX>()),
-                                  (line_min_blocks<R, N, line_batch_threads<R, DIM, N, EPBX>()>()))
+                                  (line_min_blocks<R, N, VOL, line_batch_threads<R, DIM, N, EPBX>(), NODAL>()))
 volume_batched(const VolArgs<R> *__restrict__ args, const BatchWork *__restrict__ work,
                const int *__restrict__ nwork) {
   __shared__ __align__(16) unsigned char sa[sizeof(VolArgs<R>)];
@@ -1916,7 +1922,7 @@ volume_batched(const VolArgs<R> *__restrict__ args, const BatchWork *__restrict_
     const BatchWork it = work[w];
     stage_record(sa, &args[it.item]);
     __syncthreads();
-    volume_line_body<R, DIM, N, VOL, line_batch_threads<R, DIM, N, EPBX>(), Shape<DIM, N, EPBX>::EPB>(
+    volume_line_body<R, DIM, N, VOL, line_batch_threads<R, DIM, N, EPBX>(), Shape<DIM, N, EPBX>::EPB, NODAL>(
         *reinterpret_cast<const VolArgs<R> *>(sa), it.block);
   }
 }
@@ -2011,14 +2017,14 @@ static __global__ void island_faces_kernel(int nf, int epb, const int *__restric
   if (flag[face_elem[2 * f] / epb] || flag[face_elem[2 * f + 1] / epb]) list[atomicAdd(count, 1)] = f;
 }
 
-template <typename R, int DIM, int N, int VOL>
+template <typename R, int DIM, int N, int VOL, bool NODAL>
 __global__ void __launch_bounds__((line_batch_threads<R, DIM, N, 0>()),
-                                  (line_min_blocks<R, N, line_batch_threads<R, DIM, N, 0>()>()))
+                                  (line_min_blocks<R, N, VOL, line_batch_threads<R, DIM, N, 0>(), NODAL>()))
 volume_list_kernel(const VolArgs<R> a, const int *__restrict__ list, const int *__restrict__ count) {
   const int n = *count;
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
     __syncthreads();  // the previous block's shared memory is free
-    volume_line_body<R, DIM, N, VOL, line_batch_threads<R, DIM, N, 0>(), Shape<DIM, N>::EPB>(a, list[w]);
+    volume_line_body<R, DIM, N, VOL, line_batch_threads<R, DIM, N, 0>(), Shape<DIM, N>::EPB, NODAL>(a, list[w]);
   }
 }
 

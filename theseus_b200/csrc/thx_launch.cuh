@@ -64,16 +64,17 @@ cudaError_t launch_volume_lte(const VolArgs<double> &a, cudaStream_t s, int prep
                       s, a);
 }
 
-// The line kernel (ideal gas): one thread per tensor line.
-template <typename R, int DIM, int N, int VOL, int T = kLineThreads>
+// The line kernel (ideal gas): one thread per tensor line.  NODAL: for meshes
+// whose metric varies within the element.
+template <typename R, int DIM, int N, int VOL, bool NODAL, int T = kLineThreads>
 cudaError_t launch_volume_line(const VolArgs<R> &a, cudaStream_t s, int prepare) {
   using S = LineShape<DIM, N, T>;
-  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T>::bytes();
+  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T, 0, NODAL>::bytes();
   if (prepare)
-    return cudaFuncSetAttribute(volume_line_kernel<R, DIM, N, VOL, T>,
+    return cudaFuncSetAttribute(volume_line_kernel<R, DIM, N, VOL, T, NODAL>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (a.ne <= 0) return cudaSuccess;
-  volume_line_kernel<R, DIM, N, VOL, T><<<(a.ne + S::EPB - 1) / S::EPB, T, smem, s>>>(a);
+  volume_line_kernel<R, DIM, N, VOL, T, NODAL><<<(a.ne + S::EPB - 1) / S::EPB, T, smem, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -205,18 +206,18 @@ cudaError_t launch_lte_temperature(const double *u, long long L, const LteDev &t
   return launch_early(lte_temperature_kernel<DIM>, grid, 256, 0, s, u, L, t, Tn, Cn, status);
 }
 
-template <typename R, int DIM, int N, int VOL, int EPBX = 0>
+template <typename R, int DIM, int N, int VOL, bool NODAL, int EPBX = 0>
 cudaError_t launch_volume_batched(const VolArgs<R> *args, const BatchWork *work, const int *nwork,
                                   int grid, cudaStream_t s, int prepare) {
   constexpr int T = line_batch_threads<R, DIM, N, EPBX>();
-  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T, Shape<DIM, N, EPBX>::EPB>::bytes();
+  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T, Shape<DIM, N, EPBX>::EPB, NODAL>::bytes();
   if (prepare)
-    return cudaFuncSetAttribute(volume_batched<R, DIM, N, VOL, EPBX>,
+    return cudaFuncSetAttribute(volume_batched<R, DIM, N, VOL, NODAL, EPBX>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (grid <= 0) return cudaSuccess;
   // the tuned grid counts CTAs of Shape's threads; this kernel's are smaller
   constexpr int scale = Shape<DIM, N, EPBX>::THREADS / T;
-  volume_batched<R, DIM, N, VOL, EPBX><<<grid * scale, T, smem, s>>>(args, work, nwork);
+  volume_batched<R, DIM, N, VOL, NODAL, EPBX><<<grid * scale, T, smem, s>>>(args, work, nwork);
   return cudaGetLastError();
 }
 
@@ -270,15 +271,15 @@ template <typename R>
 using FaceListLaunch = cudaError_t (*)(const FaceArgs<R> &, const int *, cudaStream_t);
 constexpr int kIslandGrid = 148 * 4;
 
-template <typename R, int DIM, int N, int VOL>
+template <typename R, int DIM, int N, int VOL, bool NODAL>
 cudaError_t launch_volume_list(const VolArgs<R> &a, const int *list, const int *count, cudaStream_t s,
                                int prepare) {
   constexpr int T = line_batch_threads<R, DIM, N, 0>();
-  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T, Shape<DIM, N>::EPB>::bytes();
+  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T, Shape<DIM, N>::EPB, NODAL>::bytes();
   if (prepare)
-    return cudaFuncSetAttribute(volume_list_kernel<R, DIM, N, VOL>,
+    return cudaFuncSetAttribute(volume_list_kernel<R, DIM, N, VOL, NODAL>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  volume_list_kernel<R, DIM, N, VOL><<<kIslandGrid, T, smem, s>>>(a, list, count);
+  volume_list_kernel<R, DIM, N, VOL, NODAL><<<kIslandGrid, T, smem, s>>>(a, list, count);
   return cudaGetLastError();
 }
 
@@ -335,21 +336,21 @@ cudaError_t launch_blend(const BlendArgs<R> &a, cudaStream_t s) {
 
 template <typename R>
 struct OrderKernelsT {
-  VolLaunch<R> vol[4];           // [volume flux]
+  VolLaunch<R> vol[4][2];        // [volume flux][metric varies within the element]
   SmallLaunch<R> small[4][2];    // smaller meshes [volume flux][face terms too]
   VolLaunch<R> vol_tma[4];       // bulk-copy-staged
   GradLaunch<R> grad;
   GradLineLaunch<R> grad_line;   // axis-aligned meshes
   BlendLaunch<R> blend;
   VolLaunch<R> fv;               // subcell FV rate of blended elements
-  VolBatchLaunch<R> volb[4];     // [volume flux]
+  VolBatchLaunch<R> volb[4][2];  // as vol
   GradBatchLaunch<R> gradb;
   // half-size CTAs (epb_half elements each; 0 and null when EPB is 1)
   int epb, epb_half;
-  VolBatchLaunch<R> volb_half[4];
+  VolBatchLaunch<R> volb_half[4][2];
   GradBatchLaunch<R> gradb_half;
   // FP64 islands (Euler, blending; set in the FP64 units only)
-  VolListLaunch<R> voll[4];      // [volume flux]
+  VolListLaunch<R> voll[4][2];   // as vol
   VolListLaunch<R> fvl;
   BlendListLaunch<R> blendl;
 };

@@ -193,7 +193,7 @@ extern "C" int thx_rhs_euler_noalloc(const thx_geometry *g, const thx_config *cf
                                                             : VOL_CENTRAL;
   VolLaunch<double> vol = nullptr;
 #define THX_NOALLOC_PICK(P, D, NN) \
-  if (dim == D && N == NN) vol = order_kernels_##P##_##D##_##NN().vol[vk];
+  if (dim == D && N == NN) vol = order_kernels_##P##_##D##_##NN().vol[vk][1];
   THX_FOR_ORDERS(THX_NOALLOC_PICK, 0, 2)
   THX_FOR_ORDERS(THX_NOALLOC_PICK, 0, 3)
 #undef THX_NOALLOC_PICK
@@ -202,7 +202,7 @@ extern "C" int thx_rhs_euler_noalloc(const thx_geometry *g, const thx_config *cf
   VolArgs<double> va{};
   va.u = u; va.du = dudt; va.ne = ne;
   va.jac = g->jac; va.jac_es = nd; va.jac_ns = 1;
-  va.met = g->metric; va.met_es = (long long)nd * dim * dim; va.met_ns = dim * dim;
+  va.met = g->metric; va.met_es = (long long)nd * dim * dim; va.met_ns = dim * dim; va.met_cs = 1;
   va.elem_face = elem_face; va.fstar = fstar;
   va.wm = g->face_wminus; va.wp = g->face_wplus; va.w_fs = nfp; va.w_ps = 1;
   va.nf_int = nf; va.bw = nullptr;  // periodic: every face is interior

@@ -53,7 +53,8 @@ using HostRing = StagingRing<CudaStaging>;
 
 // Strides of the (possibly compressed) geometry arrays on the device.
 struct Layout {
-  long long jac_es = 0, jac_ns = 0, met_es = 0, met_ns = 0;
+  long long jac_es = 0, jac_ns = 0, met_es = 0;
+  int met_ns = 0, met_cs = 1;
   long long n_fs = 0, n_ps = 0, w_fs = 0, w_ps = 0;
   long long sub_es[3] = {0, 0, 0};
 };

@@ -134,10 +134,10 @@ __device__ __forceinline__ void small_body(const VolArgs<R> &a, const FaceArgs<R
       B[k] = sP[(el * PRIM + k) * ND + nb];
     }
     // one metric row per element: 0.5*(m+m) == m
-    const R *m = a.met + (long long)(e0 + el) * a.met_es + dir * DIM;
+    const R *m = a.met + (long long)(e0 + el) * a.met_es + dir * DIM * a.met_cs;
 #pragma unroll
     for (int d = 0; d < DIM; ++d)
-      met[d] = a.met_ns == 0 ? m[d] : R(0.5) * (m[(long long)na * a.met_ns + d] + m[(long long)nb * a.met_ns + d]);
+      met[d] = a.met_ns == 0 ? m[d] : R(0.5) * (m[na * a.met_ns + d * a.met_cs] + m[nb * a.met_ns + d * a.met_cs]);
     if (FASTABLE && slow) pair_flux<R, DIM, VOL, false, LM_BRANCH>(a.gas, A, B, met, F);
     else pair_flux<R, DIM, VOL, FASTABLE, LM_BRANCH>(a.gas, A, B, met, F);
 #pragma unroll

@@ -42,13 +42,15 @@ struct LineShape {
 // more CTAs per SM).
 constexpr int kLineThreads = 128;
 
-template <typename R, int DIM, int N, int VOL, int T, int EPBX = 0>
+// NODAL: the metric varies within the element and is read from memory;
+// otherwise one metric per element, staged.
+template <typename R, int DIM, int N, int VOL, int T, int EPBX = 0, bool NODAL = false>
 struct LineSmem {
   using S = LineShape<DIM, N, T, EPBX>;
   static constexpr int PRIM = node_fields<R, DIM, VOL>();
   static constexpr int FIELDS = PRIM + S::NEQ;
   static constexpr int OPS = (N * N + 1) / 2 * 2;
-  static constexpr int MET = (S::EPB * DIM * DIM + 1) / 2 * 2;  // one metric per element
+  static constexpr int MET = NODAL ? 0 : (S::EPB * DIM * DIM + 1) / 2 * 2;
   static constexpr size_t bytes() {
     return sizeof(R) * ((size_t)OPS + MET + (size_t)FIELDS * S::FS) + sizeof(int) * S::EPB * 2 * DIM;
   }
@@ -380,12 +382,13 @@ __device__ __forceinline__ void lift_and_store(const VolArgs<R> &a, const int e,
 }
 
 // One CTA's work: elements [block*EPB, block*EPB + EPB).  su: the block's
-// state staged in shared memory (array k at k*kstride), or nullptr.
-template <typename R, int DIM, int N, int VOL, int T, int EPBX = 0>
+// state staged in shared memory (array k at k*kstride), or nullptr.  Without
+// NODAL the metric must be one per element (met_ns == 0).
+template <typename R, int DIM, int N, int VOL, int T, int EPBX = 0, bool NODAL = false>
 __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int block, const R *su = nullptr,
                                                  const int kstride = 0) {
   using S = LineShape<DIM, N, T, EPBX>;
-  using M = LineSmem<R, DIM, N, VOL, T, EPBX>;
+  using M = LineSmem<R, DIM, N, VOL, T, EPBX, NODAL>;
   constexpr int ND = S::ND, NEQ = S::NEQ, EPB = S::EPB, NL = S::NL, FS = S::FS, PRIM = M::PRIM;
   constexpr bool FASTABLE = !IsF32<R>::value && (VOL == VOL_CHANDRASHEKAR || VOL == VOL_RANOCHA);
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -416,9 +419,10 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
   }
   for (int i = tid; i < N * N; i += T) sD[i] = a.ops[i];
   for (int i = tid; i < nodes / ND * 2 * DIM; i += T) sF[i] = a.elem_face[(long long)e0 * 2 * DIM + i];
-  if (a.met_ns == 0)
+  if constexpr (!NODAL) {
     for (int i = tid; i < nodes / ND * DIM * DIM; i += T)
       sM[i] = a.met[(long long)(e0 + i / (DIM * DIM)) * a.met_es + i % (DIM * DIM)];
+  }
   bool slow = false;
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
@@ -472,29 +476,29 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
     bool straight = !active || ((!FASTABLE || !slow) && series_line<R, DIM, N, VOL, FS>(a.gas, sP, base, stride));
     straight = __all_sync(0xffffffffu, straight);
     if (active) {  // the barrier between the directions is every thread's
-    const R *mrow = a.met + (long long)e * a.met_es + dir * DIM;
-    R met[DIM];
-    if (a.met_ns == 0) {
+    const R *mrow = a.met + (long long)e * a.met_es + dir * DIM * a.met_cs;
+    // metric row of the line's node i
+    auto row = [&](int i, R *m) {
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) met[d] = sM[(el * DIM + dir) * DIM + d];
-    }
+      for (int d = 0; d < DIM; ++d) {
+        if constexpr (NODAL) m[d] = mrow[line_node<DIM, N>(dir, line, i) * a.met_ns + d * a.met_cs];
+        else m[d] = sM[(el * DIM + dir) * DIM + d];
+      }
+    };
+    R met[DIM];
+    if constexpr (!NODAL) row(0, met);
     auto load = [&](int s, R *P) {
 #pragma unroll
       for (int k = 0; k < PRIM; ++k) P[k] = sP[k * FS + s];
     };
-    // averaged metric row of a pair (one row per element: 0.5*(m+m) == m)
-    auto pair_met = [&](int i, int j, R *m) {
-      if (a.met_ns != 0) {
-        const R *ma = mrow + (long long)line_node<DIM, N>(dir, line, i) * a.met_ns;
-        const R *mb = mrow + (long long)line_node<DIM, N>(dir, line, j) * a.met_ns;
+    // averaged metric row of node j and a node with row mi (one row per
+    // element: 0.5*(m+m) == m)
+    auto pair_met = [&](const R *mi, int j, R *m) {
+      if constexpr (NODAL) row(j, m);
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) m[d] = R(0.5) * (ma[d] + mb[d]);
-      } else {
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) m[d] = met[d];
-      }
+      for (int d = 0; d < DIM; ++d) m[d] = NODAL ? R(0.5) * (mi[d] + m[d]) : mi[d];
     };
-    if (straight && a.met_ns == 0) {
+    if (straight) {
       // unrolled, the sums in registers: no branch separates the pairs, so
       // that several are in flight
       R acc[N][NEQ];
@@ -506,11 +510,13 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
       for (int i = 0; i < N - 1; ++i) {
         R A[PRIM];
         load(base + i * stride, A);
+        if constexpr (NODAL) row(i, met);
 #pragma unroll
         for (int j = i + 1; j < N; ++j) {
-          R B[PRIM], F[NEQ];
+          R B[PRIM], m[DIM], F[NEQ];
           load(base + j * stride, B);
-          pair_flux<R, DIM, VOL, FASTABLE, LM_SERIES>(a.gas, A, B, met, F);
+          pair_met(met, j, m);
+          pair_flux<R, DIM, VOL, FASTABLE, LM_SERIES>(a.gas, A, B, m, F);
           const R ci = sD[i * N + j], cj = sD[j * N + i];
 #pragma unroll
           for (int k = 0; k < NEQ; ++k) {
@@ -537,6 +543,7 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
         const int si = base + i * stride;
         R A[PRIM], sum[NEQ];
         load(si, A);
+        if constexpr (NODAL) row(i, met);
 #pragma unroll
         for (int k = 0; k < NEQ; ++k) sum[k] = sR[k * FS + si];
         auto pairs = [&](auto shared) {
@@ -545,7 +552,7 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
             const int sj = base + j * stride;
             R B[PRIM], m[DIM], F[NEQ];
             load(sj, B);
-            pair_met(i, j, m);
+            pair_met(met, j, m);
             pair_flux<R, DIM, VOL, decltype(shared)::value, LM_BRANCH>(a.gas, A, B, m, F);
             const R ci = sD[i * N + j], cj = sD[j * N + i];
 #pragma unroll
@@ -602,14 +609,14 @@ constexpr int line_threads() {
 // 32^3 p=4 (N = 5): FP64 three CTAs of 128 threads 0.337 ms, four (spills)
 // 0.357, two 0.390; FP32 five 0.171, six (spills) 0.172, four 0.177.  At 40^3
 // p=3 (N = 4) FP64: four 0.437 ms, three 0.441.
-template <typename R, int N, int T>
+template <typename R, int N, int VOL, int T, bool NODAL = false>
 constexpr int line_min_blocks() {
-  return (IsF32<R>::value ? 5 : N >= 5 ? 3 : 4) * 128 / T;
+  return (IsF32<R>::value ? 5 : VOL == VOL_CENTRAL && N >= 6 && NODAL ? 2 : N >= 5 ? 3 : 4) * 128 / T;
 }
 
-template <typename R, int DIM, int N, int VOL, int T>
-__global__ void __launch_bounds__(T, (line_min_blocks<R, N, T>())) volume_line_kernel(const VolArgs<R> a) {
-  volume_line_body<R, DIM, N, VOL, T>(a, blockIdx.x);
+template <typename R, int DIM, int N, int VOL, int T, bool NODAL>
+__global__ void __launch_bounds__(T, (line_min_blocks<R, N, VOL, T, NODAL>())) volume_line_kernel(const VolArgs<R> a) {
+  volume_line_body<R, DIM, N, VOL, T, 0, NODAL>(a, blockIdx.x);
 }
 
 }  // namespace thx
