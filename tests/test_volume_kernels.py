@@ -163,3 +163,31 @@ def test_metric_per_node(cuda, dim, order):
         compare(m, nearly, ns, **kw)
     m.metric[...] = m.metric[:1]
     compare(m, smooth_state(m, seed=order), True, numerical_flux="ranocha", surface_flux="hll", mu=0.03)
+
+
+@pytest.mark.parametrize("dim,order", sorted(SIZES))
+@pytest.mark.parametrize("size", [0, 1, 2])
+def test_fp32_sizes(cuda, dim, order, size):
+    """FP32-mixed on the same meshes.  Euler, neighbouring nodes' densities and
+    pressures up to 8 % apart: a rate sums differences of fluxes that a few
+    roundings of 6e-8 each enter, 3e-7 of the rate at most where every
+    logarithmic mean is as good (bar 5e-7; means from the rounded ratio's
+    logarithm are off by 1e-6).  Navier-Stokes on boxes along the axes: the bar
+    of the FP32 right-hand sides, 2e-5."""
+    import torch
+    m = box(dim, order, SIZES[dim, order][size])
+
+    def error(u, ns, vol, surf, **kw):
+        off = [float(u[k].mean()) for k in range(dim + 2)]
+        o = np.array(off).reshape(-1, 1, 1)
+        u = (u - o).astype(np.float32).astype(np.float64) + o  # what the working copy holds
+        op = (T.NSOperator if ns else T.EulerOperator)(m, numerical_flux=vol, surface_flux=surf, precision="fp32",
+                                                       state_offset=off, **kw)
+        ud = to_dev(u, torch.float64)
+        du = op.Mult(ud, torch.empty_like(ud)).cpu().numpy()
+        cfg = T.make_config(flow="ns" if ns else "euler", volume_flux=vol, surface_flux=surf, **kw)
+        return rel_l2(du, O.rhs(oracle_mesh(m), cfg, u, nthreads=O.max_threads())).max()
+
+    for vol, surf in (("ranocha", "llf"), ("chandrashekar", "roe"), ("hll", "hll")):
+        assert error(rough_state(m, order, 1.08), False, vol, surf) <= 5e-7, (vol, surf)
+    assert error(smooth_state(m, seed=order), True, "ranocha", "hll", mu=0.01) <= 2e-5

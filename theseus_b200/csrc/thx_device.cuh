@@ -137,17 +137,21 @@ __device__ __forceinline__ double log_mean(double x, double y) {
 }
 // FP32 path: the same function with f = (xi-1)/(xi+1) = (y-x)/(y+x) formed
 // directly (one division; y-x is exact for near-equal arguments) and
-// u = f^2.  The near-equal series is evaluated in FP64: its argument u < 1e-4
-// only scales corrections of relative size u/3, so it is formed in FP32; and
-// with eps = u (35 + u (21 + 15 u)) / 105 <= 3.4e-5, 52.5 / (105 (1 + eps)) =
-// (1 - eps + eps^2) / 2 to a relative 4e-14, far below the FP32 result's
-// rounding, without an FP64 division.
+// u = f^2.  The near-equal series is evaluated in FP64: its argument u only
+// scales corrections of relative size u/3, so it is formed in FP32; and with
+// eps = u (35 + u (21 + 15 u)) / 105, 52.5 / (105 (1 + eps)) = (1 - eps +
+// eps^2) / 2, without an FP64 division.  It serves up to u = 2.5e-3 (ratios
+// below 1.105), where it is good to 6e-10 and the closed form, whose rounded
+// ratio's logarithm is small, only to about 1e-6; up to the reference's 1e-4 the
+// lines of smooth flows on coarse meshes left the straight path of the volume
+// kernel.
+constexpr float kSeriesF32 = 2.5e-3f;
 template <int MODE = LM_BRANCH>
 __device__ __forceinline__ float log_mean(float x, float y) {
   const float s = x + y, d = y - x;
   const float f = fdiv(d, s);
   const float u = f * f;
-  if (MODE == LM_SERIES || u < 1e-4f) {
+  if (MODE == LM_SERIES || u < kSeriesF32) {
     const double ud = u;
     const double eps = ud * (35.0 + ud * (21.0 + 15.0 * ud)) * (1.0 / 105.0);
     return s * (float)(0.5 * (1.0 - eps + eps * eps));

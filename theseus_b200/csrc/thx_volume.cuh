@@ -174,7 +174,8 @@ __device__ __forceinline__ void pair_flux(const GasT<R> &g, const R *A, const R 
 
 // Whether every logarithmic mean between the nodes of a line takes its
 // series: the largest ratio of its arguments over the line stays below the
-// branch's (ratio 1.0202 for ((r-1)/(r+1))^2 < 1e-4, 1.666 for 1/16).
+// branch's (ratio 1.0202 for ((r-1)/(r+1))^2 < 1e-4 in FP64, 1.105 for 2.5e-3
+// in FP32, 1.666 for 1/16 in the perturbation form).
 template <typename R, int DIM, int N, int VOL, int FS>
 __device__ __forceinline__ bool series_line(const GasT<R> &g, const R *sP, int base, int stride) {
   if (VOL != VOL_CHANDRASHEKAR && VOL != VOL_RANOCHA) return true;
@@ -195,7 +196,7 @@ __device__ __forceinline__ bool series_line(const GasT<R> &g, const R *sP, int b
       hi[q] = x > hi[q] ? x : hi[q];
     }
   }
-  const R bound = pert ? R(1.65) : R(1.0195);
+  const R bound = pert ? R(1.65) : IsF32<R>::value ? R(1.10) : R(1.0195);
   if (VOL == VOL_RANOCHA) return lo[0] > R(0) && lo[1] > R(0) && hi[0] * hi[1] < bound * (lo[0] * lo[1]);
   return lo[0] > R(0) && lo[1] > R(0) && hi[0] < bound * lo[0] && hi[1] < bound * lo[1];
 }
