@@ -567,7 +567,8 @@ typedef struct {
   int32_t active_cases;
   int32_t tuned;          /* 1 once every axis has been searched */
   int32_t volume_grid, face_grid, gradient_grid;  /* the best so far */
-  int32_t elements_per_block;  /* of the best configuration */
+  int32_t elements_per_block;  /* of the best configuration: blocks of a thread per
+                                  node; the volume kernel's are its own */
   double best_cost_ms;    /* cost of the best grids on the axis being searched
                              (-1 before its first timing) */
 } thx_engine_group;

@@ -236,3 +236,22 @@ def test_engine_metric_per_node(cuda, precision):
             assert np.array_equal(got, ref)
         else:
             assert field_errors(got, ref, c.mesh.dim).max() <= 1e-5
+
+
+@pytest.mark.parametrize("dim,order,n", [(2, 2, (9, 9)), (2, 5, (7, 6)), (3, 2, (5, 4, 5))])
+def test_engine_fp32_result_independent_of_the_tuner(cuda, dim, order, n):
+    """The tuner's search tries the block sizes on real launches, at times that
+    depend on the load.  Vortices whose steepest lines take the logarithm of the
+    far means and whose others take its series: their bits must not show it."""
+    def run(others):
+        batch = [vortex_case(dim, order, n, False, 240, strength=5.0, seed=7)]
+        batch += [vortex_case(dim, order, n, False, 240, strength=4.0, seed=30 + i) for i in range(others)]
+        for c in batch:
+            c.state_offset = (0.0,) * 5
+        eng = BatchEngine(precision="fp32", steps_per_launch=3, **FLUX)
+        out = run_engine(eng, batch)[0]
+        eng.close()
+        return out
+    first = run(0)
+    for others in (0, 15, 60):
+        assert np.array_equal(first, run(others)), others

@@ -89,8 +89,10 @@ template <typename R>
 struct Group {
   int dim = 0, N = 0;
   bool ns = false, nodal = false;
-  int epb = 1, nfp = 1;  // epb: elements per CTA of the current tables
-  int epb_full = 1, epb_half = 0;
+  int nfp = 1;
+  bool half = false;  // the current tables are those of the half-size CTAs
+  // elements per work item, full and half size: gradient, volume
+  int epb_full = 1, epb_half = 0, vepb_full = 1, vepb_half = 0;
   std::vector<EngineCase *> cases;
   // admitted cases whose set-up may still run on the set-up stream: they join
   // `cases` once their ready event has completed, so a group's launches never
@@ -102,9 +104,9 @@ struct Group {
   VolArgs<R> *dvol = nullptr;
   FaceArgs<R> *dface = nullptr;
   GradArgs<R> *dgrad = nullptr;
-  BatchWork *dwv = nullptr, *dwf = nullptr;
-  int *dcount = nullptr;  // [0] volume/gradient work, [1] face work
-  int cap_cases = 0, cap_wv = 0, cap_wf = 0;
+  BatchWork *dwv = nullptr, *dwf = nullptr, *dwg = nullptr;
+  int *dcount = nullptr;  // [0] volume, [1] face, [2] gradient work
+  int cap_cases = 0, cap_wv = 0, cap_wf = 0, cap_wg = 0;
   // pinned staging of the tables, a ring of three: with at most two launches
   // queued, the copies out of the slot about to be refilled have finished,
   // so a rewrite does not wait for the GPU (with the engine lock held)
@@ -565,7 +567,6 @@ class Engine final : public EngineBase {
     pick_kernels(*G, vk, ns);
     if (!G->volb || !G->faceb || !G->gradb) return THX_ERR_UNSUPPORTED;
     if (G->epb_half > 0 && (!G->volb_half || !G->gradb_half)) return THX_ERR_UNSUPPORTED;
-    G->epb = G->epb_full;
     if (G->volb(nullptr, nullptr, nullptr, 0, nullptr, 1) != cudaSuccess ||
         G->gradb(nullptr, nullptr, nullptr, 0, nullptr, 1) != cudaSuccess ||
         (G->epb_half > 0 && (G->volb_half(nullptr, nullptr, nullptr, 0, nullptr, 1) != cudaSuccess ||
@@ -601,6 +602,7 @@ class Engine final : public EngineBase {
     cudaFree(G.dface);
     cudaFree(G.dgrad);
     cudaFree(G.dwv);
+    cudaFree(G.dwg);
     cudaFree(G.dwf);
     cudaFree(G.dcount);
     for (int i = 0; i < Group<R>::kStaging; ++i) {
@@ -618,12 +620,14 @@ class Engine final : public EngineBase {
   // Rewrite the group's argument tables and work lists (between launches).
   int upload_tables(Group<R> &G) {
     const int nc = (int)G.cases.size();
-    int nwv = 0, nwf = 0;
+    const int vepb = G.half ? G.vepb_half : G.vepb_full, gepb = G.half ? G.epb_half : G.epb_full;
+    int nwv = 0, nwf = 0, nwg = 0;
     for (EngineCase *c : G.cases) {
-      nwv += (c->h->ne + G.epb - 1) / G.epb;
+      nwv += (c->h->ne + vepb - 1) / vepb;
+      if (G.ns) nwg += (c->h->ne + gepb - 1) / gepb;
       nwf += (int)(((long long)c->h->nf * G.nfp + kFaceBlock - 1) / kFaceBlock);
     }
-    bool grow = nc > G.cap_cases || nwv > G.cap_wv || nwf > G.cap_wf;
+    bool grow = nc > G.cap_cases || nwv > G.cap_wv || nwf > G.cap_wf || nwg > G.cap_wg;
     if (grow) {
       // Stream-ordered reallocation on the group's stream: the old tables are
       // freed after the launches in flight that read them, and nothing here
@@ -634,8 +638,9 @@ class Engine final : public EngineBase {
       const int cc = nc > G.cap_cases ? grow_to(nc, G.cap_cases) : G.cap_cases;
       const int cv = nwv > G.cap_wv ? grow_to(nwv, G.cap_wv) : G.cap_wv;
       const int cf = nwf > G.cap_wf ? grow_to(nwf, G.cap_wf) : G.cap_wf;
-      void *old[5] = {G.dvol, G.dface, G.dgrad, G.dwv, G.dwf};
-      G.dvol = nullptr; G.dface = nullptr; G.dgrad = nullptr; G.dwv = nullptr; G.dwf = nullptr;
+      const int cg = nwg > G.cap_wg ? grow_to(nwg, G.cap_wg) : G.cap_wg;
+      void *old[6] = {G.dvol, G.dface, G.dgrad, G.dwv, G.dwf, G.dwg};
+      G.dvol = nullptr; G.dface = nullptr; G.dgrad = nullptr; G.dwv = nullptr; G.dwf = nullptr; G.dwg = nullptr;
       if (G.exec) {
         cudaGraphExecDestroy(G.exec);
         G.exec = nullptr;
@@ -649,18 +654,20 @@ class Engine final : public EngineBase {
           !get((void **)&G.dface, sizeof(FaceArgs<R>) * 3 * cc) ||
           !get((void **)&G.dgrad, sizeof(GradArgs<R>) * 3 * cc) ||
           !get((void **)&G.dwv, sizeof(BatchWork) * cv) || !get((void **)&G.dwf, sizeof(BatchWork) * cf) ||
-          (!G.dcount && !get((void **)&G.dcount, sizeof(int) * 2))) {
-        G.cap_cases = G.cap_wv = G.cap_wf = 0;
+          (cg && !get((void **)&G.dwg, sizeof(BatchWork) * cg)) ||
+          (!G.dcount && !get((void **)&G.dcount, sizeof(int) * 3))) {
+        G.cap_cases = G.cap_wv = G.cap_wf = G.cap_wg = 0;
         return cuda_failed(cudaGetLastError(), "cudaMallocFromPoolAsync(group tables)", THX_ERR_OUT_OF_MEMORY);
       }
       G.cap_cases = cc;
       G.cap_wv = cv;
+      G.cap_wg = cg;
       G.cap_wf = cf;
     }
     const size_t bv = sizeof(VolArgs<R>) * 3 * nc, bf = sizeof(FaceArgs<R>) * 3 * nc;
     const size_t bg = sizeof(GradArgs<R>) * 3 * nc;
-    const size_t bw = sizeof(BatchWork) * (size_t)(nwv + nwf);
-    const size_t need = bv + bf + bg + bw + 2 * sizeof(int) + 64;
+    const size_t bw = sizeof(BatchWork) * (size_t)(nwv + nwf + nwg);
+    const size_t need = bv + bf + bg + bw + 3 * sizeof(int) + 64;
     const int slot = G.stage_pos;
     THX_CU(cudaEventSynchronize(G.staged[slot]));  // this slot's last copies are done
     if (need > G.staging_bytes[slot]) {
@@ -682,7 +689,7 @@ class Engine final : public EngineBase {
     GradArgs<R> *hg = reinterpret_cast<GradArgs<R> *>(stg + bv + bf);
     BatchWork *hw = reinterpret_cast<BatchWork *>(stg + bv + bf + bg);
     int *hc = reinterpret_cast<int *>(stg + bv + bf + bg + bw);
-    int wv = 0, wf = 0;
+    int wv = 0, wf = 0, wg = 0;
     for (int i = 0; i < nc; ++i) {
       EngineCase *c = G.cases[i];
       thx_operator_s *h = c->h;
@@ -693,8 +700,9 @@ class Engine final : public EngineBase {
         std::memcpy(&hf[j], pk + sizeof(VolArgs<R>), sizeof(FaceArgs<R>));
         std::memcpy(&hg[j], pk + sizeof(VolArgs<R>) + sizeof(FaceArgs<R>), sizeof(GradArgs<R>));
       }
-      const int nb = (h->ne + G.epb - 1) / G.epb;
+      const int nb = (h->ne + vepb - 1) / vepb, ng = G.ns ? (h->ne + gepb - 1) / gepb : 0;
       for (int b = 0; b < nb; ++b) hw[wv++] = BatchWork{i, b};
+      for (int b = 0; b < ng; ++b) hw[nwv + nwf + wg++] = BatchWork{i, b};
     }
     for (int i = 0; i < nc; ++i) {
       thx_operator_s *h = G.cases[i]->h;
@@ -703,6 +711,7 @@ class Engine final : public EngineBase {
     }
     hc[0] = nwv;
     hc[1] = nwf;
+    hc[2] = nwg;
     // the argument records of stage s start at s*nc; the graph indexes
     // tables by capacity, so place each stage block at s*cap
     for (int stage = 0; stage < 3; ++stage) {
@@ -716,10 +725,11 @@ class Engine final : public EngineBase {
     }
     if ((nwv && cudaMemcpyAsync(G.dwv, hw, sizeof(BatchWork) * nwv, cudaMemcpyHostToDevice, G.stream) != cudaSuccess) ||
         (nwf && cudaMemcpyAsync(G.dwf, hw + nwv, sizeof(BatchWork) * nwf, cudaMemcpyHostToDevice, G.stream) != cudaSuccess) ||
-        cudaMemcpyAsync(G.dcount, hc, sizeof(int) * 2, cudaMemcpyHostToDevice, G.stream) != cudaSuccess ||
+        (nwg && cudaMemcpyAsync(G.dwg, hw + nwv + nwf, sizeof(BatchWork) * nwg, cudaMemcpyHostToDevice, G.stream) != cudaSuccess) ||
+        cudaMemcpyAsync(G.dcount, hc, sizeof(int) * 3, cudaMemcpyHostToDevice, G.stream) != cudaSuccess ||
         cudaEventRecord(G.staged[slot], G.stream) != cudaSuccess)
       return cuda_failed(cudaGetLastError(), "work list upload");
-    table_bytes_ += (int64_t)(bv + bf + bg + bw + 2 * sizeof(int));
+    table_bytes_ += (int64_t)(bv + bf + bg + bw + 3 * sizeof(int));
     G.stage_pos = (slot + 1) % Group<R>::kStaging;
     G.nwv = nwv;
     G.nodes = 0;
@@ -743,7 +753,7 @@ class Engine final : public EngineBase {
     for (int step = 0; step < k_ && e == cudaSuccess; ++step)
       for (int stage = 0; stage < 3 && e == cudaSuccess; ++stage) {
         const size_t o = (size_t)stage * G.cap_cases;
-        if (G.ns) e = gradb(G.dgrad + o, G.dwv, G.dcount, gg, G.stream, 0);
+        if (G.ns) e = gradb(G.dgrad + o, G.dwg, G.dcount + 2, gg, G.stream, 0);
         if (e == cudaSuccess) e = G.faceb(G.dface + o, G.dwf, G.dcount + 1, gf, G.stream, 0);
         if (e == cudaSuccess) e = volb(G.dvol + o, G.dwv, G.dcount, grid, G.stream, 0);
       }
@@ -871,9 +881,8 @@ class Engine final : public EngineBase {
       grids = G.exec_grids;
     }
     // the work lists follow the CTA size
-    const int epb = grids.half ? G.epb_half : G.epb_full;
-    if (epb != G.epb) {
-      G.epb = epb;
+    if (grids.half != G.half) {
+      G.half = grids.half;
       G.dirty = true;
     }
     const double ta = now();
@@ -947,6 +956,8 @@ void Engine<double>::pick_kernels(Group<double> &G, int vk, int ns) {
     G.gradb = k.gradb;                                      \
     G.epb_full = k.epb;                                     \
     G.epb_half = k.epb_half;                                \
+    G.vepb_full = k.vepb;                                   \
+    G.vepb_half = k.vepb_half;                              \
     G.volb_half = k.volb_half[vk][G.nodal];                 \
     G.gradb_half = k.gradb_half;                            \
   }
@@ -966,6 +977,8 @@ void Engine<float>::pick_kernels(Group<float> &G, int vk, int ns) {
     G.gradb = k.gradb;                                      \
     G.epb_full = k.epb;                                     \
     G.epb_half = k.epb_half;                                \
+    G.vepb_full = k.vepb;                                   \
+    G.vepb_half = k.vepb_half;                              \
     G.volb_half = k.volb_half[vk][G.nodal];                 \
     G.gradb_half = k.gradb_half;                            \
   }

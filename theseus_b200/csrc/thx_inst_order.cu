@@ -25,8 +25,8 @@ THX_TYPE(THX_PREC) THX_NAME(THX_PREC, THX_DIM, THX_N)() {
   k.small[V][0] = &launch_volume_small<R, THX_DIM, THX_N, V, false>; \
   k.small[V][1] = &launch_volume_small<R, THX_DIM, THX_N, V, true>;  \
   k.vol_tma[V] = &launch_volume_tma<R, THX_DIM, THX_N, V>;     \
-  k.volb[V][0] = &launch_volume_batched<R, THX_DIM, THX_N, V, false>; \
-  k.volb[V][1] = &launch_volume_batched<R, THX_DIM, THX_N, V, true>;
+  k.volb[V][0] = &launch_volume_batched<R, THX_DIM, THX_N, V, false, batch_threads<R, THX_DIM, THX_N>()>; \
+  k.volb[V][1] = &launch_volume_batched<R, THX_DIM, THX_N, V, true, batch_threads<R, THX_DIM, THX_N>()>;
   THX_SETV(VOL_CHANDRASHEKAR)
   THX_SETV(VOL_RANOCHA)
   THX_SETV(VOL_PIROZZOLI)
@@ -43,20 +43,21 @@ THX_TYPE(THX_PREC) THX_NAME(THX_PREC, THX_DIM, THX_N)() {
   k.gradb = &launch_grad_batched<R, THX_DIM, THX_N>;
   k.epb = Shape<THX_DIM, THX_N>::EPB;
   k.epb_half = half_epb<THX_DIM, THX_N>();
+  k.vepb = LineShape<THX_DIM, THX_N, batch_threads<R, THX_DIM, THX_N>()>::EPB;
+  k.vepb_half = k.epb_half;
   for (auto &row : k.volb_half)
     for (auto &v : row) v = nullptr;
   k.gradb_half = nullptr;
   if constexpr (half_epb<THX_DIM, THX_N>() > 0) {
     constexpr int H = half_epb<THX_DIM, THX_N>();
-    // FP64: the line and the pair kernel give the same bits.  FP32 may contract
-    // multiply-adds differently in the two, and a case's result must not depend
-    // on what the tuner finds for the cases beside it.
+    // FP64: the line and the pair kernel give the same bits
 #if THX_PREC == 0
 #define THX_SETH(V) k.volb_half[V][0] = k.volb_half[V][1] = &launch_volume_batched_pairs<R, THX_DIM, THX_N, V, H>;
 #else
-#define THX_SETH(V)                                                          \
-  k.volb_half[V][0] = &launch_volume_batched<R, THX_DIM, THX_N, V, false, H>; \
-  k.volb_half[V][1] = &launch_volume_batched<R, THX_DIM, THX_N, V, true, H>;
+    k.vepb_half = k.vepb;
+#define THX_SETH(V)                      \
+  k.volb_half[V][0] = k.volb[V][0];      \
+  k.volb_half[V][1] = k.volb[V][1];
 #endif
     THX_SETH(VOL_CHANDRASHEKAR)
     THX_SETH(VOL_RANOCHA)

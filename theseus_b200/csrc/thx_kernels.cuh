@@ -1905,14 +1905,21 @@ __device__ __forceinline__ void stage_record(unsigned char *dst, const A *src) {
   for (int i = threadIdx.x; i < (int)(sizeof(A) / 8); i += blockDim.x) d[i] = s[i];
 }
 
-// Line kernel over a work list; EPBX (0: Shape's) elements per work item.
-template <typename R, int DIM, int N, int EPBX>
-constexpr int line_batch_threads() {
-  return line_threads<DIM, N, Shape<DIM, N, EPBX>::EPB>();
+// Line kernel over a work list, T threads and LineShape's elements per work
+// item.  (Elements counted for a thread per node instead left a third of the
+// threads without a line at p=2 and p=5.)  64 threads, which balance better, where
+// all of them have a line (FP32: seven eighths), otherwise 128: 64 cases of 6^3
+// p=3, FP64, 151 against 157 us a stage; of 24^2 p=5 169 against 153.  FP32 has
+// no second size: which lines share a warp decides which of the body's two
+// paths they take, in FP32 those may differ in the last bit, and a case's result
+// must not depend on the size that the tuner finds for the cases beside it.
+template <typename R, int DIM, int N>
+constexpr int batch_threads() {
+  constexpr int NL = DIM == 2 ? N : N * N;
+  return 64 / NL * NL >= (IsF32<R>::value ? 56 : 64) ? 64 : 128;
 }
-template <typename R, int DIM, int N, int VOL, bool NODAL, int EPBX = 0>
-__global__ void __launch_bounds__((line_batch_threads<R, DIM, N, EPBX>()),
-                                  (line_min_blocks<R, N, VOL, line_batch_threads<R, DIM, N, EPBX>(), NODAL>()))
+template <typename R, int DIM, int N, int VOL, bool NODAL, int T>
+__global__ void __launch_bounds__(T, (line_min_blocks<R, N, VOL, T, NODAL>()))
 volume_batched(const VolArgs<R> *__restrict__ args, const BatchWork *__restrict__ work,
                const int *__restrict__ nwork) {
   __shared__ __align__(16) unsigned char sa[sizeof(VolArgs<R>)];
@@ -1922,8 +1929,7 @@ volume_batched(const VolArgs<R> *__restrict__ args, const BatchWork *__restrict_
     const BatchWork it = work[w];
     stage_record(sa, &args[it.item]);
     __syncthreads();
-    volume_line_body<R, DIM, N, VOL, line_batch_threads<R, DIM, N, EPBX>(), Shape<DIM, N, EPBX>::EPB, NODAL>(
-        *reinterpret_cast<const VolArgs<R> *>(sa), it.block);
+    volume_line_body<R, DIM, N, VOL, T, 0, NODAL>(*reinterpret_cast<const VolArgs<R> *>(sa), it.block);
   }
 }
 
@@ -2017,14 +2023,17 @@ static __global__ void island_faces_kernel(int nf, int epb, const int *__restric
   if (flag[face_elem[2 * f] / epb] || flag[face_elem[2 * f + 1] / epb]) list[atomicAdd(count, 1)] = f;
 }
 
+template <int DIM, int N>
+constexpr int line_list_threads() {
+  return line_threads<DIM, N, Shape<DIM, N>::EPB>();
+}
 template <typename R, int DIM, int N, int VOL, bool NODAL>
-__global__ void __launch_bounds__((line_batch_threads<R, DIM, N, 0>()),
-                                  (line_min_blocks<R, N, VOL, line_batch_threads<R, DIM, N, 0>(), NODAL>()))
+__global__ void __launch_bounds__((line_list_threads<DIM, N>()), (line_min_blocks<R, N, VOL, line_list_threads<DIM, N>(), NODAL>()))
 volume_list_kernel(const VolArgs<R> a, const int *__restrict__ list, const int *__restrict__ count) {
   const int n = *count;
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
     __syncthreads();  // the previous block's shared memory is free
-    volume_line_body<R, DIM, N, VOL, line_batch_threads<R, DIM, N, 0>(), Shape<DIM, N>::EPB, NODAL>(a, list[w]);
+    volume_line_body<R, DIM, N, VOL, line_list_threads<DIM, N>(), Shape<DIM, N>::EPB, NODAL>(a, list[w]);
   }
 }
 

@@ -5,6 +5,7 @@
 #include "thx_bc.cuh"
 
 #include <algorithm>
+#include <atomic>
 
 namespace thx {
 
@@ -206,18 +207,23 @@ cudaError_t launch_lte_temperature(const double *u, long long L, const LteDev &t
   return launch_early(lte_temperature_kernel<DIM>, grid, 256, 0, s, u, L, t, Tn, Cn, status);
 }
 
-template <typename R, int DIM, int N, int VOL, bool NODAL, int EPBX = 0>
+// grid: in units of the CTAs that are resident at once on an SM; more than all
+// of them balance the items better.
+template <typename R, int DIM, int N, int VOL, bool NODAL, int T>
 cudaError_t launch_volume_batched(const VolArgs<R> *args, const BatchWork *work, const int *nwork,
                                   int grid, cudaStream_t s, int prepare) {
-  constexpr int T = line_batch_threads<R, DIM, N, EPBX>();
-  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T, Shape<DIM, N, EPBX>::EPB, NODAL>::bytes();
-  if (prepare)
-    return cudaFuncSetAttribute(volume_batched<R, DIM, N, VOL, NODAL, EPBX>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kern = volume_batched<R, DIM, N, VOL, NODAL, T>;
+  constexpr size_t smem = LineSmem<R, DIM, N, VOL, T, 0, NODAL>::bytes();
+  static std::atomic<int> resident{0};  // CTAs per SM
+  if (prepare) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, T, smem);
+    resident = per;
+    return e;
+  }
   if (grid <= 0) return cudaSuccess;
-  // the tuned grid counts CTAs of Shape's threads; this kernel's are smaller
-  constexpr int scale = Shape<DIM, N, EPBX>::THREADS / T;
-  volume_batched<R, DIM, N, VOL, NODAL, EPBX><<<grid * scale, T, smem, s>>>(args, work, nwork);
+  kern<<<grid * std::max(1, resident.load()), T, smem, s>>>(args, work, nwork);
   return cudaGetLastError();
 }
 
@@ -274,7 +280,7 @@ constexpr int kIslandGrid = 148 * 4;
 template <typename R, int DIM, int N, int VOL, bool NODAL>
 cudaError_t launch_volume_list(const VolArgs<R> &a, const int *list, const int *count, cudaStream_t s,
                                int prepare) {
-  constexpr int T = line_batch_threads<R, DIM, N, 0>();
+  constexpr int T = line_list_threads<DIM, N>();
   constexpr size_t smem = LineSmem<R, DIM, N, VOL, T, Shape<DIM, N>::EPB, NODAL>::bytes();
   if (prepare)
     return cudaFuncSetAttribute(volume_list_kernel<R, DIM, N, VOL, NODAL>,
@@ -345,8 +351,9 @@ struct OrderKernelsT {
   VolLaunch<R> fv;               // subcell FV rate of blended elements
   VolBatchLaunch<R> volb[4][2];  // as vol
   GradBatchLaunch<R> gradb;
-  // half-size CTAs (epb_half elements each; 0 and null when EPB is 1)
-  int epb, epb_half;
+  // half-size CTAs (null when the gradient's full-size CTA holds one element)
+  int epb, epb_half;             // elements per work item of the gradient kernels
+  int vepb, vepb_half;           // of the volume kernels
   VolBatchLaunch<R> volb_half[4][2];
   GradBatchLaunch<R> gradb_half;
   // FP64 islands (Euler, blending; set in the FP64 units only)
