@@ -278,3 +278,49 @@ def test_oracle_stability_boundary_term_is_active():
     mp = bmesh(2, 3, (4, 3), {}, periodic=(True, True), perturb=False)
     _, periodic = O.estimate_dt(oracle_mesh(mp), cfg, u, 1.0)
     assert with_b[1] > periodic[1]
+
+
+# the kernels of larger meshes on a small one (volume_staging=1), and meshes of
+# their sizes, in both dimensions
+BOX_WALLS = [(2, 2, (4, 5), 1), (2, 3, (5, 4), 1), (2, 4, (3, 4), 1), (2, 5, (3, 3), 1), (3, 2, (3, 4, 3), 1),
+             (3, 3, (3, 2, 3), 1), (3, 4, (2, 3, 2), 1), (3, 5, (2, 2, 3), 1), (2, 3, (97, 95), 0), (3, 3, (13, 12, 13), 0)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,order,n,staging", BOX_WALLS)
+@pytest.mark.parametrize("name", NS_CONDITIONS)
+def test_gpu_ns_walls_on_boxes(cuda, dim, order, n, staging, name):
+    """Navier-Stokes boundaries of boxes along the axes, where the gradient is
+    formed line by line: the boundary lift at the ends of the lines and the
+    boundary points' primitive gradients, at faces, edges and corners."""
+    import torch
+    sides = {f"{'xyz'[d]}{s}": spec(name, dim) for d in range(dim) for s in "-+"}
+    m = bmesh(dim, order, n, sides, perturb=False)
+    u = smooth_state(m, seed=order)
+    op = T.NSOperator(m, numerical_flux="ranocha", surface_flux="hll", mu=0.01, Pr=0.72, volume_staging=staging)
+    ud = torch.as_tensor(u, device="cuda")
+    du = torch.empty_like(ud)
+    op.Mult(ud, du)
+    cfg = T.make_config(flow="ns", volume_flux="ranocha", surface_flux="hll", mu=0.01, Pr=0.72)
+    ref = O.rhs(oracle_mesh(m), cfg, u, nthreads=O.max_threads())
+    assert rel_l2(du.cpu().numpy(), ref).max() <= TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,order,n", [(2, 3, (5, 4)), (3, 4, (2, 3, 2))])
+def test_gpu_ns_mirrored_boxes(cuda, dim, order, n):
+    """Boxes along the axes whose metric has another sign and size from element
+    to element, with a wall."""
+    import torch
+    m = bmesh(dim, order, n, {"x-": spec("no-slip-adiabatic", dim), "x+": spec("no-slip-adiabatic", dim)}, perturb=False)
+    rng = np.random.default_rng(3)
+    for d in range(dim):
+        m.metric[:, :, d, d] *= (rng.choice([-1.0, 1.0], m.num_elements) * rng.uniform(0.5, 2.0, m.num_elements))[:, None]
+    m.jac[...] *= rng.choice([-1.0, 1.0], m.num_elements)[:, None]
+    u = smooth_state(m, seed=order)
+    op = T.NSOperator(m, numerical_flux="ranocha", surface_flux="hll", mu=0.01, Pr=0.72, volume_staging=1)
+    ud = torch.as_tensor(u, device="cuda")
+    du = op.Mult(ud, torch.empty_like(ud))
+    cfg = T.make_config(flow="ns", volume_flux="ranocha", surface_flux="hll", mu=0.01, Pr=0.72)
+    ref = O.rhs(oracle_mesh(m), cfg, u, nthreads=O.max_threads())
+    assert rel_l2(du.cpu().numpy(), ref).max() <= TOL

@@ -238,14 +238,15 @@ def test_engine_metric_per_node(cuda, precision):
             assert field_errors(got, ref, c.mesh.dim).max() <= 1e-5
 
 
-@pytest.mark.parametrize("dim,order,n", [(2, 2, (9, 9)), (2, 5, (7, 6)), (3, 2, (5, 4, 5))])
-def test_engine_fp32_result_independent_of_the_tuner(cuda, dim, order, n):
+@pytest.mark.parametrize("viscous", [False, True])
+@pytest.mark.parametrize("dim,order,n", [(2, 2, (9, 9)), (2, 5, (7, 6)), (3, 2, (5, 4, 5)), (3, 4, (3, 3, 3))])
+def test_engine_fp32_result_independent_of_the_tuner(cuda, dim, order, n, viscous):
     """The tuner's search tries the block sizes on real launches, at times that
     depend on the load.  Vortices whose steepest lines take the logarithm of the
     far means and whose others take its series: their bits must not show it."""
     def run(others):
-        batch = [vortex_case(dim, order, n, False, 240, strength=5.0, seed=7)]
-        batch += [vortex_case(dim, order, n, False, 240, strength=4.0, seed=30 + i) for i in range(others)]
+        batch = [vortex_case(dim, order, n, viscous, 240, strength=5.0, seed=7)]
+        batch += [vortex_case(dim, order, n, viscous, 240, strength=4.0, seed=30 + i) for i in range(others)]
         for c in batch:
             c.state_offset = (0.0,) * 5
         eng = BatchEngine(precision="fp32", steps_per_launch=3, **FLUX)
