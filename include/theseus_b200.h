@@ -554,10 +554,13 @@ int thx_engine_fetch(thx_engine e, int64_t id, double *u_host);
 int thx_engine_get_stats(thx_engine e, thx_engine_stats *out);
 
 /* One batch group of the engine (cases of the same dimension, order and
- * flow model share persistent batched kernels and one CUDA graph).  The
- * engine tunes those kernels online by coordinate search: the elements per
- * CTA of the volume and gradient kernels (as many as fit 256 threads, or
- * half as many), then the volume grid over {1,2,4} x SMs, the face grid over
+ * flow model, and with the metric constant or varying within the elements,
+ * share persistent batched kernels and one CUDA graph).  The engine tunes
+ * those kernels online by coordinate search: the elements per CTA of the
+ * gradient kernels and, in FP64, the form of the volume kernel (as many as fit
+ * 256 threads and a thread per tensor line, or half as many and a thread per
+ * pair), then the volume grid over {1,2,4} x SMs, each standing for the CTAs
+ * that are resident there at once, the face grid over
  * {4,8,16} x SMs and (Navier-Stokes) the gradient grid over {1,2,4} x SMs,
  * each candidate timed with CUDA events around two launches that advance real
  * cases (the better one counts); cost = device milliseconds per (solution

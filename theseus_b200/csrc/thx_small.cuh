@@ -16,8 +16,8 @@ constexpr int kSmallThreads = 256;
 constexpr int kSmallSMs = 148;
 
 // Elements per CTA.  With the face terms: spread over the SMs, up to about two
-// pairs per thread.  Without: over the CTAs that are resident at once, three
-// per SM in FP64 and four in FP32, up to a node per thread.
+// pairs per thread.  Without: over three CTAs per SM in FP64 and four in FP32
+// (see small_mesh), up to a node per thread.
 __host__ constexpr int small_epb(int dim, int N, int ne, bool faces, bool f32) {
   const int nd = dim == 2 ? N * N : N * N * N;
   const int pairs = dim * (nd / N) * (N * (N - 1) / 2);
@@ -30,12 +30,16 @@ __host__ constexpr int small_epb(int dim, int N, int ne, bool faces, bool f32) {
 
 // Which volume kernel a mesh takes: 2 this one with the face terms, 1 this one
 // after the face kernel, 0 the line kernel after the face kernel.  The first
-// two while their CTAs are resident at once (two, and three or four per SM, by
-// their registers); beyond, the line kernel's fewer instructions outweigh its longer
-// chains.  RK3 stage of the 2-D Euler vortex, FP64, first / second / line
-// kernel: 32^2 p=3 9.8 / 13.7 / 21.6 us, 48^2 10.3 / 14.4 / 22.0, 64^2 16.4 /
-// 15.8 / 22.2, 96^2 28.7 / 24.1 / 22.6, 128^2 44.3 / 32.8 / 28.5; 3-D p=3 5^3
-// 10.3 / 16.4 / 28.7, 7^3 18.5 / 16.4 / 28.7, 16^3 110 / 85 / 51.
+// two up to two, and three or four, CTAs per SM, which their registers allow at
+// once; beyond, the line kernel's fewer instructions outweigh its longer chains.
+// RK3 stage, Euler FP64, first / second / line kernel: 2-D p=3 32^2 7.6 / 9.8 /
+// 19.0 us, 48^2 8.8 / 10.8 / 17.6, 64^2 14.8 / 13.9 / 18.3, 96^2 27.1 / 19.6 /
+// 21.0, 128^2 41.2 / 30.7 / 28.4; 3-D p=3 5^3 8.6 / 11.7 / 25.2, 7^3 15.5 / 13.5 /
+// 26.9, 16^3 103 / 52 / 50.  Shared memory holds only two FP64 CTAs of the second
+// per SM at 3-D p=5, and at 3-D p=4 with all fluxes but Ranocha's: the last of
+// three then run in a second wave, with which the kernel still beats the line
+// kernel (p=5 441 elements 35.6 / 46.9 us Ranocha; p=4 840 elements 28.6 / 41.4
+// Chandrashekar), except with the central flux (27.1 / 22.9, 25.3 / 23.0).
 __host__ constexpr int small_mesh(int dim, int N, int ne, bool f32) {
   const int e2 = small_epb(dim, N, ne, true, f32), e1 = small_epb(dim, N, ne, false, f32);
   return (ne + e2 - 1) / e2 <= 2 * kSmallSMs ? 2 : (ne + e1 - 1) / e1 <= (f32 ? 4 : 3) * kSmallSMs ? 1 : 0;

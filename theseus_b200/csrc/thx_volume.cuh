@@ -1,14 +1,14 @@
 // thx_volume.cuh -- flux-differencing volume kernel of the ideal gas: one
 // thread per tensor line.
 //
-// What bounds it: the arithmetic pipes (FP64: 59 % of the pipe's cycles at
-// 20^3 p=4, with 44 % of the issue slots; FP32: 64 % of the issue slots).  A
+// What bounds it: the arithmetic pipes (FP64: 60 % of the pipe's cycles at
+// 20^3 p=4, with 43 % of the issue slots; FP32: 64 % of the issue slots).  A
 // thread owns a line of N nodes: it evaluates the line's N(N-1)/2 symmetric
 // pairs once each and adds every pair flux to its two end nodes.  Against one
 // thread per pair, with the fluxes passed through shared memory to one thread
 // per node (15 shared-memory accesses and their index arithmetic per pair),
 // it executes a third of the instructions: at 32^3 p=4 Ranocha, with the
-// shared reciprocals below, 0.712 -> 0.337 ms in FP64 and 0.370 -> 0.171 ms
+// shared reciprocals below, 0.712 -> 0.357 ms in FP64 and 0.370 -> 0.179 ms
 // FP32-mixed (less the viscous divergence, which the gradient kernel forms).
 // Pairs run in (lower, upper) lexicographic order, so every node receives its
 // terms in the order of the other end's index, as
@@ -38,8 +38,8 @@ struct LineShape {
   static constexpr int FS = EPB * NDP;     // stride of a field
 };
 
-// Threads per CTA of the line kernels: 128 (3-D: 3 to 14 elements; four or
-// more CTAs per SM).
+// Threads per CTA of the line kernels: 128 (3-D: 3 to 14 elements; three or
+// more CTAs per SM, see line_min_blocks).
 constexpr int kLineThreads = 128;
 
 // NODAL: the metric varies within the element and is read from memory;
@@ -607,9 +607,11 @@ constexpr int line_threads() {
 }
 
 // Resident CTAs of T threads per SM that the registers are bounded for.  At
-// 32^3 p=4 (N = 5): FP64 three CTAs of 128 threads 0.337 ms, four (spills)
-// 0.357, two 0.390; FP32 five 0.171, six (spills) 0.172, four 0.177.  At 40^3
-// p=3 (N = 4) FP64: four 0.437 ms, three 0.441.
+// 32^3 p=4 (N = 5), relative: FP64 three CTAs of 128 threads 1, four (spills)
+// 1.06, two 1.16; FP32 five 1, six (spills) 1.01, four 1.04.  At 40^3 p=3
+// (N = 4) FP64: four 1, three 1.01.  With a metric per node at p=5 (N = 6) the
+// central flux spills at three: 16^3 Euler stage 254 us, 192 at two (the other
+// fluxes, slower per pair: Ranocha 247 at three, 291 at two).
 template <typename R, int N, int VOL, int T, bool NODAL = false>
 constexpr int line_min_blocks() {
   return (IsF32<R>::value ? 5 : VOL == VOL_CENTRAL && N >= 6 && NODAL ? 2 : N >= 5 ? 3 : 4) * 128 / T;
