@@ -8,7 +8,7 @@
 // thread per pair, with the fluxes passed through shared memory to one thread
 // per node (15 shared-memory accesses and their index arithmetic per pair),
 // it executes a third of the instructions: at 32^3 p=4 Ranocha, with the
-// shared reciprocals below, 0.712 -> 0.357 ms in FP64 and 0.370 -> 0.179 ms
+// shared reciprocals below, 0.712 -> 0.357 ms in FP64 and 0.370 -> 0.171 ms
 // FP32-mixed (less the viscous divergence, which the gradient kernel forms).
 // Pairs run in (lower, upper) lexicographic order, so every node receives its
 // terms in the order of the other end's index, as
@@ -473,21 +473,21 @@ __device__ __forceinline__ void volume_line_body(const VolArgs<R> &a, const int 
     int base, stride;
     line_base<DIM, N, S::LS>(dir, line, base, stride);
     base += el * S::NDP;
+    // one metric per element: its row, loaded with the values of the test below
+    // (after the vote it delayed the pairs: 32^3 p=4 FP32 179 -> 171 us)
+    R met[DIM];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) met[d] = !NODAL && active ? sM[(el * DIM + dir) * DIM + d] : R(0);
     // straight-line pairs if every line of the warp's allows them
     bool straight = !active || ((!FASTABLE || !slow) && series_line<R, DIM, N, VOL, FS>(a.gas, sP, base, stride));
     straight = __all_sync(0xffffffffu, straight);
     if (active) {  // the barrier between the directions is every thread's
     const R *mrow = a.met + (long long)e * a.met_es + dir * DIM * a.met_cs;
-    // metric row of the line's node i
+    // NODAL: metric row of the line's node i
     auto row = [&](int i, R *m) {
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) {
-        if constexpr (NODAL) m[d] = mrow[line_node<DIM, N>(dir, line, i) * a.met_ns + d * a.met_cs];
-        else m[d] = sM[(el * DIM + dir) * DIM + d];
-      }
+      for (int d = 0; d < DIM; ++d) m[d] = mrow[line_node<DIM, N>(dir, line, i) * a.met_ns + d * a.met_cs];
     };
-    R met[DIM];
-    if constexpr (!NODAL) row(0, met);
     auto load = [&](int s, R *P) {
 #pragma unroll
       for (int k = 0; k < PRIM; ++k) P[k] = sP[k * FS + s];
