@@ -256,3 +256,14 @@ def test_engine_fp32_result_independent_of_the_tuner(cuda, dim, order, n, viscou
     first = run(0)
     for others in (0, 15, 60):
         assert np.array_equal(first, run(others)), others
+
+
+def test_engine_admits_a_state_larger_than_half_the_ring(cuda):
+    """An FP32 working copy of 132 MiB, which the upload ring of 256 MiB takes in
+    two pieces."""
+    c = vortex_case(2, 5, (490, 490), False, 2)
+    eng = BatchEngine(precision="fp32", steps_per_launch=2, **FLUX)
+    got = run_engine(eng, [c])[0]
+    eng.close()
+    assert np.abs(got - c.u0).max() > 0
+    assert field_errors(got, alone(c, "fp32"), 2).max() <= 1e-7
